@@ -242,8 +242,7 @@ def _prepare_raster(c, seed):
     return state
 
 
-def _prepare_tonemap(c, seed):
-    torch.ops.load_library(build.TORCH_OP_LIB)
+def _tonemap_inputs(c, seed):
     g = _generator(seed)
     B, w, h = c["batch"], c["w"], c["h"]
     # exposed frames: smooth shading with grain, darks near 0 and highlights that clip
@@ -256,10 +255,16 @@ def _prepare_tonemap(c, seed):
     response = (torch.linspace(0, 1, c["bins"], device=DEV) ** (1 / 2.2)).repeat(1, 3, 1).contiguous()
     leaves = dict(x=x, exposures=ev, white_balance=wb, vignette=torch.tensor([0.1, -0.05, 0.01], device=DEV),
                   centre=torch.zeros((1, 2, 1, 1), device=DEV), response=response)
+    return leaves, torch.randn((B, 3, h, w), device=DEV, generator=g)
+
+
+def _prepare_tonemap(c, seed):
+    torch.ops.load_library(build.TORCH_OP_LIB)
+    leaves, grad = _tonemap_inputs(c, seed)
     for v in leaves.values():
         v.requires_grad_(True)
-    return dict(kind="tonemap", leaves=leaves, frames=torch.arange(B, device=DEV, dtype=torch.int32), size=(w, h), leak=c["leak"],
-                grad=torch.randn((B, 3, h, w), device=DEV, generator=g))
+    return dict(kind="tonemap", leaves=leaves, frames=torch.arange(c["batch"], device=DEV, dtype=torch.int32), size=(c["w"], c["h"]),
+                leak=c["leak"], grad=grad)
 
 
 def _prepare_preprocess(c, seed):
@@ -363,3 +368,45 @@ def tolerance(case):
     # float32 sums of up to millions of terms in the GPU's order. Seen between the same pass twice, and between the pass over
     # the recorded lists and the one over all points: rel up to 2.4e-6 (intrinsics gradient), max up to 1.3e-5 (environment map).
     return {"rel": 1e-5, "max": 6e-5}
+
+
+# ---- the same numbers in 64 bits ----------------------------------------------------------------------------------------
+def _exact_tonemap(c, seed):
+    leaves, grad = _tonemap_inputs(c, seed)
+    a = {k: v.double().requires_grad_(True) for k, v in leaves.items()}
+    B, w, h, K, leak = c["batch"], c["w"], c["h"], c["bins"], c["leak"]
+    yy, xx = torch.meshgrid(torch.linspace(-1, 1, h, device=DEV, dtype=torch.float64), torch.linspace(-1, 1, w, device=DEV, dtype=torch.float64),
+                            indexing="ij")
+    images, grads = [], None
+    for b in range(B):      # an image at a time: eight bytes a value, and several values a pixel
+        du, dv = (xx - a["centre"][0, 0, 0, 0]) * (w / h), yy - a["centre"][0, 1, 0, 0]
+        r2 = du * du + dv * dv
+        vig = a["vignette"]
+        v = (1 + r2 * (vig[0] + r2 * (vig[1] + r2 * vig[2]))) * (a["white_balance"][b] * (a["x"][b] * torch.exp2(-a["exposures"][b])))
+        z = v.detach()
+        t = z.clamp(0, 1) * (K - 1)
+        i0 = t.floor().long()
+        fr = t - i0
+        row = torch.arange(3, device=DEV).view(3, 1, 1) * K
+        lo, hi = row + i0, row + (i0 + 1).clamp(max=K - 1)
+        curve = a["response"].detach().reshape(-1)
+        out = curve[lo] * (1 - fr) + curve[hi] * fr
+        slope = (curve[hi] - curve[lo]) * (K - 1) * ((z > 0) & (z < 1))
+        if leak > 0:
+            knee = z.abs() + 1e-4
+            out = out + torch.where(z < 0, leak * z, torch.where(z > 1, leak - leak * knee ** -0.5, 0.0))
+            slope = slope + torch.where(z < 0, leak, torch.where(z > 1, 0.5 * leak * knee ** -1.5, 0.0))
+        images.append(out)
+        up = grad[b].double()
+        part = list(torch.autograd.grad(v, [a[k] for k in ("x", "exposures", "white_balance", "vignette", "centre")], up * slope))
+        bins = torch.bincount(lo.reshape(-1), (up * (1 - fr)).reshape(-1), 3 * K) + torch.bincount(hi.reshape(-1), (up * fr).reshape(-1), 3 * K)
+        part.append(bins.view_as(a["response"]))
+        grads = part if grads is None else [p + q for p, q in zip(grads, part)]
+    return dict(image=torch.stack(images), grad=grads)
+
+
+def exact(case, seed):
+    """The tonemapper in 64 bits. The rasterizer has no such value: which pixel a point rounds to and whether it passes the depth
+    test are decided on float32 numbers, and 64-bit ones decide some of them differently, which moves whole splats. The
+    preprocessing's results are permutations and float32 distances that are compared bit by bit."""
+    return _exact_tonemap(case, seed) if case["kind"] == "tonemap" else None
