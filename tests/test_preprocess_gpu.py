@@ -148,6 +148,28 @@ def test_knn_distance_equals_all_pairs(cuda_lib, n, k, shape):
     assert np.array_equal(got, _knn_brute_force(xyz, k))
 
 
+@pytest.mark.parametrize("n,shape", [(9, "line"), (4097, "line"), (6000, "clusters"), (5000, "far"), (3000, "duplicates")])
+def test_knn_distance_in_uneven_surroundings(cuda_lib, n, shape):
+    """Dense and sparse surroundings in one cloud, in random order: queries that settle in the cells next to theirs and
+    queries that grow their cube give the exact value."""
+    rng = np.random.default_rng(n)
+    if shape == "line":
+        xyz = np.zeros((n, 3))
+        xyz[:, 0] = rng.uniform(0, 1, n) ** 3
+    elif shape == "clusters":
+        xyz = rng.uniform(-1, 1, (n, 3))
+        xyz[: n // 2] = rng.normal(0, 0.004, (n // 2, 3)) + rng.choice([-0.5, 0.5], (n // 2, 1))
+    elif shape == "far":
+        xyz = rng.uniform(0, 1, (n, 3)) + np.array([1000.0, -2000.0, 500.0])
+    else:
+        xyz = np.repeat(rng.uniform(-1, 1, (n // 3, 3)), 3, axis=0)
+    xyz = rng.permutation(xyz.astype(np.float32))
+    pos = np.zeros((xyz.shape[0], 4), np.float32)
+    pos[:, :3] = xyz
+    got = preprocess.knn_distance(torch.from_numpy(pos).cuda(), k=4).cpu().numpy()
+    assert np.array_equal(got, _knn_brute_force(xyz, 4))
+
+
 def test_knn_distance_against_a_kd_tree(cuda_lib):
     """300 k points on surfaces (the benchmark's scene generator): scipy's KD-tree in float64 as the second opinion."""
     from scipy.spatial import cKDTree
