@@ -268,10 +268,14 @@ constexpr int kListUnusable = kVisibleSegments + 2, kListConsumed = kVisibleSegm
 #endif
 
 // Large region of a full workspace (behind the camera records and pixel records).
-// Forward: candidate streams - the depth prepass leaves, per view of its group of up to four, the points that landed inside
-// the image as (x, y, depth, point id) records, one segment per block, so that the blend kernel neither reads the
+// Forward: candidate streams - the depth prepass leaves, per view of its group of up to four, the points that can still be
+// accepted as (x, y, depth, point id) records, one segment per block, so that the blend kernel neither reads the
 // positions again nor projects a second time.
 constexpr int kCandViews = 4;
+// With the radius drop-out rule in use, the id word of a record is id | (layers the rule leaves - 1) << 28: clouds of more
+// than kCandIdMask points then go without candidate streams.
+constexpr int kCandLayerShift = 28, kCandIdMask = (1 << kCandLayerShift) - 1;
+static_assert(kMaxLayers <= 8, "three bits hold the layer count");
 struct LargeRegion
 {
     size_t cand_rec, cand_count, total;  // byte offsets from the region's start (forward)

@@ -139,17 +139,29 @@ static adop_scene make_scene(RenderInfo& info, const Tensor& texture, const Tens
 static size_t ensure_workspace(RenderInfo& info, const std::vector<adop_view>& views, int64_t num_layers, const adop_scene& sc,
                                const torch::TensorOptions& opt, bool forward)
 {
-    // Candidate streams (adop_raster_workspace_bytes_full) pay for views of the omnidirectional model, whose projection is
-    // expensive and whose image holds a small part of the cloud; on pinhole training views they measured slower.
-    bool ocam = false;
-    for (const adop_view& v : views) ocam = ocam || v.camera_model == ADOP_CAMERA_OCAM;
-    const size_t need = (forward && ocam)
-                            ? adop_raster_workspace_bytes_full(sc.num_points, (int32_t)views.size(), views[0].w, views[0].h, (int32_t)num_layers,
-                                                               sc.channels)
-                            : adop_raster_workspace_bytes(views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
+    // With the full workspace the depth prepass hands the points that can still be accepted to the blend kernel
+    // (adop_raster_workspace_bytes_full); where the device has no room for it, the small one does.
+    size_t need = adop_raster_workspace_bytes(views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
     TORCH_CHECK(need > 0, "invalid view size / layer count");
-    if (!info.workspace.defined() || (size_t)info.workspace.numel() < need)
-        info.workspace = torch::empty({(int64_t)need}, opt.dtype(torch::kUInt8));
+    auto provide = [&](size_t bytes)
+    {
+        if (!info.workspace.defined() || (size_t)info.workspace.numel() < bytes) info.workspace = torch::empty({(int64_t)bytes}, opt.dtype(torch::kUInt8));
+    };
+    bool full = forward;
+    if (full)
+    {
+        const size_t bytes = adop_raster_workspace_bytes_full(sc.num_points, (int32_t)views.size(), views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
+        try
+        {
+            provide(bytes);
+            need = bytes;
+        }
+        catch (const c10::OutOfMemoryError&)
+        {
+            full = false;
+        }
+    }
+    if (!full) provide(need);
     if (!info.texture_interleaved.defined() || info.texture_interleaved.size(0) != sc.num_texels || info.texture_interleaved.size(1) != sc.channels)
     {
         info.texture_interleaved = torch::empty({sc.num_texels, sc.channels}, opt);

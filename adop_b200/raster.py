@@ -123,11 +123,9 @@ class PointRasterizer:
 
     def __init__(self, device="cuda:0", interleave_descriptors=True, full_workspace=None):
         """full_workspace: True sizes the forward scratch with adop_raster_workspace_bytes_full (16 bytes per point and view
-        of a group more), which lets the depth prepass hand the projected in-image points to the blend kernel instead of the
-        blend kernel reading the cloud and projecting again; False keeps the small workspace. None (default) decides per
-        call: on for views of the omnidirectional model, whose projection is expensive and whose image holds a small part
-        of the cloud (forward pass of the 100 M point viewer configuration: a third faster), off for pinhole views, where the
-        extra stream costs more than it saves (measured on the training configuration)."""
+        of a group more), which lets the depth prepass hand the projected points that can still be accepted to the blend
+        kernel instead of the blend kernel reading the cloud and projecting again; False keeps the small workspace. None
+        (default): the full workspace, or the small one where the device has no room for it."""
         self.lib = capi.load_library()
         self.device = torch.device(device)
         self._ws = None
@@ -181,10 +179,13 @@ class PointRasterizer:
             # rendering frame after frame), so the [T,C] working copy is reused as it is
             sc = self._scene_struct(scene, refresh=refresh_descriptors)
             ch = sc.channels
-            full = self.full_workspace
-            if full is None:
-                full = any(v.camera_model == capi.CAMERA_OCAM for v in va)
-            ws = self._workspace(w, h, num_layers, ch, sc.num_points, B, full=bool(full))
+            if self.full_workspace is None:
+                try:
+                    ws = self._workspace(w, h, num_layers, ch, sc.num_points, B, full=True)
+                except torch.cuda.OutOfMemoryError:
+                    ws = self._workspace(w, h, num_layers, ch)
+            else:
+                ws = self._workspace(w, h, num_layers, ch, sc.num_points, B, full=bool(self.full_workspace))
             sizes = capi.layer_sizes(w, h, num_layers)
             if out is None:
                 f32 = dict(dtype=torch.float32, device=self.device)

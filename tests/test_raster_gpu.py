@@ -375,6 +375,49 @@ def test_small_workspace_matches_full_workspace(cuda_lib):
         close(ba[k], bb[k].cpu().numpy(), name=f"small vs full grad {k}")
 
 
+@pytest.mark.parametrize("points,size,views,layers,rule,ghost,mask", [
+    (1, (40, 24), 1, 1, False, 0, False),            # one point, one layer
+    (257, (33, 17), 3, 3, False, 0, False),          # one point past a chunk, odd planes
+    (90_011, (101, 57), 5, 4, False, 0, False),      # 15 points per pixel, two groups of views
+    (90_011, (101, 57), 5, 4, True, 0, False),       # normal test and radius rule: the record carries the layer count
+    (90_011, (101, 57), 4, 5, True, 1, False),       # dropped points stay in the stream for the visible list
+    (60_000, (64, 48), 2, 5, True, 0, True),         # drop-out decisions from the caller's mask
+])
+def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib, points, size, views, layers, rule, ghost, mask):
+    """Full workspace (the prepass drops points that already fail the depth test everywhere) against the small one (every
+    point is projected and tested again): the same depths, weights and listed points bit for bit."""
+    rng = np.random.default_rng(points + layers)
+    cfg = synth.make_config("c2", n_points=points, n_views=views, size=size, layers=layers)
+    a, params = cfg["arrays"], cfg["params"]
+    params.dropout, params.dropout_seed, params.ghost_gradients = 0.3, 17, ghost
+    if rule:
+        nrm = rng.normal(size=(points, 3))
+        nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+        q = np.round((nrm + 1) * 0.5 * 1023).astype(np.uint32)
+        a["normal"] = (q[:, 0] | (q[:, 1] << 10) | (q[:, 2] << 20)).astype(np.int32)
+        a["position"][:, 3] = rng.uniform(0.01, 0.6, points).astype(np.float32)
+        params.check_normal = params.drop_out_points_by_radius = 1
+    scene = to_scene(a)
+    dm = torch.from_numpy(rng.integers(0, 2, (views, points)).astype(np.uint8)).cuda() if mask else None
+    out = []
+    for full in (False, True):
+        fwd = PointRasterizer("cuda:0", full_workspace=full).forward(scene, cfg["views"], params, layers, dropout_mask=dm)
+        assert not bool(fwd.list_unusable().any())
+        t = fwd._tiles()
+        listed = []
+        for v in range(views):
+            row = fwd.visible[v]
+            counts = row[2056:2056 + t].tolist()
+            entries = row[2056 + (t + 3) // 4 * 4:].view(t, -1, 4)
+            listed.append([sorted(map(tuple, entries[k, :counts[k]].tolist())) for k in range(t)])
+        out.append((fwd, listed))
+    (small, small_list), (full, full_list) = out
+    for l in range(layers):
+        assert torch.equal(small.depths[l], full.depths[l]) and torch.equal(small.weights[l], full.weights[l])
+        close(small.colors[l], full.colors[l].cpu().numpy(), name=f"streams colour {l}")
+    assert small_list == full_list
+
+
 def test_backward_mode_4(oracle, cuda_lib):
     cfg = synth.make_config("c1", n_points=40_000, size=(96, 96))
     cfg["params"].test_backward_mode = 4
