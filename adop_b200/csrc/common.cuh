@@ -145,6 +145,21 @@ inline void fill_layer_dims(int w, int h, int L, LayerTable* lt)
     for (int l = L; l <= kMaxLayers; ++l) lt->rec_off[l] = off;
 }
 
+// lt of the view `view` places behind the one lt was made for: the planes of a batch follow each other
+inline LayerTable layer_table_of_view(LayerTable lt, int C, int view)
+{
+    for (int l = 0; l < lt.L; ++l)
+    {
+        const size_t skip = (size_t)view * lt.w[l] * lt.h[l];
+        if (lt.depth[l]) lt.depth[l] += skip;
+        if (lt.weight[l]) lt.weight[l] += skip;
+        if (lt.color[l]) lt.color[l] += skip * C;
+        if (lt.mask[l]) lt.mask[l] += skip;
+        if (lt.grad[l]) lt.grad[l] += skip * C;
+    }
+    return lt;
+}
+
 // One view's camera is gathered from rows of the pose / intrinsics tensors (device memory: they are trainable
 // parameters) plus the ReducedImageInfo fields of the view. A small kernel does that for a chunk of views and leaves the
 // ViewCam records at the head of the workspace; the point kernels read their view's record through a pointer. (Measured
@@ -160,7 +175,11 @@ struct CamChunkSource
     int n;
     struct View { int image_index, camera_index, camera_model, w0; float crop[5]; } v[kCamChunk];
 };
-static_assert(sizeof(ViewCam) * kCamChunk <= kCamRegionBytes, "camera region too small");
+// Behind the camera records: which rows of the pose and intrinsics tensors a view of the chunk takes (for kernels that serve
+// several views in one launch).
+struct ViewRows { int image, camera; };
+static_assert((sizeof(ViewCam) + sizeof(ViewRows)) * kCamChunk <= kCamRegionBytes, "camera region too small");
+__host__ __device__ inline ViewRows* view_rows(ViewCam* cams) { return reinterpret_cast<ViewRows*>(cams + kCamChunk); }
 inline void fill_cam_chunk(CamChunkSource* c, const adop_scene* s, const adop_view* views, int n)
 {
     c->poses = s->poses; c->intrinsics = s->intrinsics; c->intrinsics_cols = s->intrinsics_cols; c->n = n;
@@ -251,6 +270,15 @@ inline VisibleList make_visible_list(int32_t* base, int num_points, int w, int h
 }
 // ints at the head of a view's list that the forward pass clears before the blend kernel appends
 inline size_t visible_list_clear_ints(int w, int h, int num_points) { return (size_t)kVisibleHeaderInts + make_tile_table(w, h, num_points).n_tiles; }
+// the list of the view `view` places behind v's, lists being list_ints apart
+__host__ __device__ inline VisibleList list_of_view(VisibleList v, size_t list_ints, int view)
+{
+    const size_t skip = (size_t)view * list_ints;
+    v.header += skip;
+    v.tile_cur += skip;
+    v.entries = reinterpret_cast<int4*>(reinterpret_cast<int*>(v.entries) + skip);
+    return v;
+}
 #if defined(__CUDACC__)
 // screen tile of an image position (clamped into the image: positions just outside layer 0 can still land in a coarser layer)
 __device__ __forceinline__ int tile_of_position(const TileTable& tt, float x, float y)
@@ -276,20 +304,57 @@ constexpr int kCandViews = 4;
 // than kCandIdMask points then go without candidate streams.
 constexpr int kCandLayerShift = 28, kCandIdMask = (1 << kCandLayerShift) - 1;
 static_assert(kMaxLayers <= 8, "three bits hold the layer count");
+// Accumulators: the views of a group are blended and resolved in one launch each when their accumulators together fit
+// kGroupAccumBytes. Small views leave the GPU half empty one at a time; large ones evict each other's accumulators from L2.
+constexpr size_t kGroupAccumBytes = (size_t)48 << 20;
 struct LargeRegion
 {
-    size_t cand_rec, cand_count, total;  // byte offsets from the region's start (forward)
+    size_t cand_rec, cand_count, accum, total;  // byte offsets from the region's start (forward)
+    int accum_views;
 };
-inline LargeRegion large_region_layout(int num_points, int num_views)
+inline LargeRegion large_region_layout(int num_points, int num_views, size_t accum_bytes)
 {
     const int v = num_views < kCandViews ? (num_views < 1 ? 1 : num_views) : kCandViews;
     const size_t cap = entry_capacity(num_points);
     LargeRegion r;
     r.cand_rec = 0;
     r.cand_count = r.cand_rec + (size_t)v * cap * 16;
-    r.total = r.cand_count + (size_t)v * kVisibleSegments * sizeof(int) + 256;
+    r.accum = r.cand_count + (((size_t)v * kVisibleSegments * sizeof(int) + 255) & ~(size_t)255);
+    r.accum_views = 1;
+    while (r.accum_views < v && (size_t)(r.accum_views + 1) * accum_bytes <= kGroupAccumBytes) ++r.accum_views;
+    r.total = r.accum + (r.accum_views > 1 ? (size_t)r.accum_views * accum_bytes : 0) + 256;
     return r;
 }
+
+// What a call sets to a constant before its kernels add to it - accumulator, weight and depth planes, list cursors, gradient
+// tensors - goes into one launch (a call used to issue a memset or fill kernel per tensor and layer, two dozen in all; on
+// the smallest training step they were a third of its launches).
+struct FillTable
+{
+    static constexpr int kMax = 32;
+    static constexpr int kWordsPerBlock = 8192;
+    struct Entry
+    {
+        uint32_t* p;
+        unsigned long long words, stride;  // words of a row, distance from row to row
+        uint32_t value;
+        unsigned blocks_per_row, first_block;
+    };
+    int n = 0;
+    unsigned blocks = 0;
+    Entry e[kMax];
+    // rows of `words` 32-bit words, `stride` words apart
+    void add(void* p, size_t words, uint32_t value, size_t rows = 1, size_t stride = 0)
+    {
+        if (!p || words == 0 || rows == 0) return;
+        Entry& q = e[n++];
+        q.p = static_cast<uint32_t*>(p); q.words = words; q.stride = stride; q.value = value;
+        q.blocks_per_row = (unsigned)((words + kWordsPerBlock - 1) / kWordsPerBlock);
+        q.first_block = blocks;
+        blocks += q.blocks_per_row * (unsigned)rows;
+    }
+};
+adop_status launch_fills(const FillTable& t, cudaStream_t st);
 
 adop_status validate_common(const adop_scene* s, const adop_view* views, int B, const adop_render_params* rp, int L);
 int sm_count();
@@ -354,6 +419,9 @@ static __global__ void k_build_cams(CamChunkSource src, ViewCam* __restrict__ ou
     if (k >= src.n) return;
     out[k] = load_view_cam(src.poses, src.intrinsics, src.intrinsics_cols, src.v[k].image_index, src.v[k].camera_index,
                            src.v[k].camera_model, src.v[k].crop, src.v[k].w0);
+    ViewRows* rows = view_rows(out);
+    rows[k].image = src.v[k].image_index;
+    rows[k].camera = src.v[k].camera_index;
 }
 // A point's descriptor: from the interleaved [T,C] copy when the caller provides one (one or two 16-byte loads), else
 // from the C planes of the [C,T] tensor.
@@ -412,10 +480,11 @@ __device__ __forceinline__ void add_descriptor_gradient(float* __restrict__ plan
         for (int c = 0; c < C; ++c) atomicAdd(planar + (size_t)c * num_texels + ti, g[c]);
     }
 }
-__device__ __forceinline__ bool point_dropped(const KernelParams& kp, int i)
+// drop-out decision of point i in the view `view` places behind the one kp was made for; n = points of the cloud
+__device__ __forceinline__ bool point_dropped(const KernelParams& kp, int view, int n, int i)
 {
-    if (kp.dropout_mask) return kp.dropout_mask[i] == 1;
-    return dropout_decision(kp.dropout, kp.dropout_seed, (uint32_t)kp.batch_slot, (uint32_t)i);
+    if (kp.dropout_mask) return kp.dropout_mask[(size_t)view * n + i] == 1;
+    return dropout_decision(kp.dropout, kp.dropout_seed, (uint32_t)(kp.batch_slot + view), (uint32_t)i);
 }
 // chunk of round k of this block, or -1 when the round has none (the last superblocks can be short)
 __device__ __forceinline__ int scheduled_chunk(const ChunkSchedule& cs, int k)

@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pts.n; i += stride)
     {
-        const bool drop_out = point_dropped(kp, i);
+        const bool drop_out = point_dropped(kp, 0, pts.n, i);
         FetchedPoint f = fetch_point(pts, i);
         RasterPoint q;
         if (!project_for_raster(cam, f.p, f.r, f.n, f.has_normal, kp.check_normal != 0, kp.dist_cutoff, &q,

@@ -14,8 +14,6 @@
 //    cloud streams through: the blend kernel's L2 hit rate is about 40 %;
 //  * the blend kernel also lists, per 32 x 16 screen tile, the points the backward pass will visit, and the depth prepass can
 //    hand the blend kernel the projected in-image points (candidate streams) when the workspace has room for them.
-#include <cooperative_groups.h>
-
 #include <cstring>
 
 #include "common.cuh"
@@ -23,66 +21,102 @@
 namespace adop {
 
 // ------------------------------------------------------------------------------------------------------
-__global__ void k_fill(float* __restrict__ dst, size_t n, float v)
+// One block per kWordsPerBlock words of a row. Bound by the write stream; 32 KB per block keeps the launch to a few waves on
+// the largest tensors and lets the short ones (a few words to a few KB) share the launch with them.
+__global__ void __launch_bounds__(kBlock) k_fill(const __grid_constant__ FillTable t)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    size_t n4 = n / 4;
-    float4 v4 = make_float4(v, v, v, v);
-    for (size_t k = i; k < n4; k += stride) reinterpret_cast<float4*>(dst)[k] = v4;
-    for (size_t k = n4 * 4 + i; k < n; k += stride) dst[k] = v;
+    int k = 0;
+    while (k + 1 < t.n && blockIdx.x >= t.e[k + 1].first_block) ++k;
+    const FillTable::Entry& q = t.e[k];
+    const unsigned at = blockIdx.x - q.first_block, row = at / q.blocks_per_row, part = at - row * q.blocks_per_row;
+    uint32_t* const line = q.p + (size_t)row * q.stride;
+    const size_t first = (size_t)part * FillTable::kWordsPerBlock;
+    const unsigned long long left = q.words - first;
+    const unsigned n = left < FillTable::kWordsPerBlock ? (unsigned)left : FillTable::kWordsPerBlock;
+    uint32_t* p = line + first;
+    const uint32_t v = q.value;
+    // up to three words in front of the first 16-byte boundary, vectors, the rest
+    const unsigned head = min((unsigned)((16u - (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) / 4u, n);
+    if (threadIdx.x < head) p[threadIdx.x] = v;
+    uint4* p4 = reinterpret_cast<uint4*>(p + head);
+    const unsigned n4 = (n - head) / 4;
+    for (unsigned i = threadIdx.x; i < n4; i += kBlock) p4[i] = make_uint4(v, v, v, v);
+    for (unsigned i = head + 4 * n4 + threadIdx.x; i < n; i += kBlock) p[i] = v;
+}
+adop_status launch_fills(const FillTable& t, cudaStream_t st)
+{
+    if (t.blocks == 0) return ADOP_OK;
+    ADOP_LAUNCH("k_fill", st, (k_fill<<<t.blocks, kBlock, 0, st>>>(t)));
+    ADOP_CUDA_TRY(cudaGetLastError());
+    return ADOP_OK;
 }
 
-// [C,T] planes <-> [T,C] interleaved descriptors (one texel per thread; plane accesses are coalesced, interleaved
-// accesses are contiguous vectors)
+// [C,T] planes <-> [T,C] interleaved descriptors. One thread per four channels of a texel: neighbouring lanes take the channel
+// groups of one texel, then the next texel, so that a warp's vector accesses to the interleaved side are 512 contiguous
+// bytes for every channel count, and its scalar accesses to the planes are runs of 128 / C4 bytes - whole sectors up to
+// sixteen channels.
 template <int C4>  // C4 = C / 4 when C is a multiple of 4 (vector stores), 0 = any C (scalar)
-__global__ void k_texture_interleave(const float* __restrict__ in, float* __restrict__ out, int C, int T)
+__global__ void __launch_bounds__(kBlock) k_texture_interleave(const float* __restrict__ in, float* __restrict__ out, int C, int T)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
+    if (C4 > 0)
     {
-        if (C4 > 0)
+        constexpr int U = 2;  // vectors per thread and round: eight plane reads in flight
+        const size_t n = (size_t)T * C4, stride = (size_t)gridDim.x * blockDim.x;
+        for (size_t j0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j0 < n; j0 += stride * U)
         {
+            float4 v[U];
 #pragma unroll
-            for (int k = 0; k < C4; ++k)
+            for (int u = 0; u < U; ++u)
             {
-                float4 v;
-                v.x = __ldcs(in + (size_t)(4 * k + 0) * T + t); v.y = __ldcs(in + (size_t)(4 * k + 1) * T + t);
-                v.z = __ldcs(in + (size_t)(4 * k + 2) * T + t); v.w = __ldcs(in + (size_t)(4 * k + 3) * T + t);
-                reinterpret_cast<float4*>(out + (size_t)t * (4 * C4))[k] = v;
+                const size_t j = j0 + u * stride;
+                if (j >= n) break;
+                const size_t t = j / (C4 > 0 ? C4 : 1);
+                const float* src = in + (size_t)(4 * (int)(j - t * C4)) * T + t;
+                v[u].x = __ldcs(src); v[u].y = __ldcs(src + T); v[u].z = __ldcs(src + 2 * (size_t)T); v[u].w = __ldcs(src + 3 * (size_t)T);
             }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j0 + u * stride < n) reinterpret_cast<float4*>(out)[j0 + u * stride] = v[u];
         }
-        else
-            for (int c = 0; c < C; ++c) out[(size_t)t * C + c] = __ldcs(in + (size_t)c * T + t);
+        return;
     }
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
+        for (int c = 0; c < C; ++c) out[(size_t)t * C + c] = __ldcs(in + (size_t)c * T + t);
 }
 template <int C4>
-__global__ void k_texture_deinterleave(const float* __restrict__ in, float* __restrict__ out, int C, int T, int accumulate)
+__global__ void __launch_bounds__(kBlock) k_texture_deinterleave(const float* __restrict__ in, float* __restrict__ out, int C, int T, int accumulate)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
+    if (C4 > 0)
     {
-        if (C4 > 0)
+        constexpr int U = 4;
+        const size_t n = (size_t)T * C4, stride = (size_t)gridDim.x * blockDim.x;
+        for (size_t j0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j0 < n; j0 += stride * U)
         {
+            float4 v[U];
 #pragma unroll
-            for (int k = 0; k < C4; ++k)
+            for (int u = 0; u < U; ++u)
+                if (j0 + u * stride < n) v[u] = __ldcs(reinterpret_cast<const float4*>(in) + j0 + u * stride);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
             {
-                const float4 v = __ldcs(reinterpret_cast<const float4*>(in + (size_t)t * (4 * C4)) + k);
-                const float vv[4] = {v.x, v.y, v.z, v.w};
+                const size_t j = j0 + u * stride;
+                if (j >= n) break;
+                const size_t t = j / (C4 > 0 ? C4 : 1);
+                float* dst = out + (size_t)(4 * (int)(j - t * C4)) * T + t;
+                const float vv[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                {
-                    float* dst = out + (size_t)(4 * k + j) * T + t;
-                    *dst = accumulate ? *dst + vv[j] : vv[j];
-                }
+                for (int c = 0; c < 4; ++c, dst += T) *dst = accumulate ? *dst + vv[c] : vv[c];
             }
         }
-        else
-            for (int c = 0; c < C; ++c)
-            {
-                float v = __ldcs(in + (size_t)t * C + c);
-                float* dst = out + (size_t)c * T + t;
-                *dst = accumulate ? *dst + v : v;
-            }
+        return;
     }
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
+        for (int c = 0; c < C; ++c)
+        {
+            float v = __ldcs(in + (size_t)t * C + c);
+            float* dst = out + (size_t)c * T + t;
+            *dst = accumulate ? *dst + v : v;
+        }
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -110,7 +144,6 @@ struct CandOut
     size_t view_stride;   // records per view
     int seg_cap;          // records per block segment
     int keep_dropped;     // the visible list wants dropped points too (ghost-gradient mode)
-    int n_points;         // stride of the drop-out mask between views
 };
 template <int L, bool PLAIN, int V, bool CAND>
 __global__ void __launch_bounds__(kBlock, PLAIN ? 8 : 4) k_depth_prepass(PointStreams pts, ChunkSchedule sched, const ViewCam* __restrict__ camp, KernelParams kp,
@@ -194,9 +227,7 @@ __global__ void __launch_bounds__(kBlock, PLAIN ? 8 : 4) k_depth_prepass(PointSt
             }
             if (CAND)
             {
-                if (keep && !co.keep_dropped)
-                    keep = kp.dropout_mask ? kp.dropout_mask[(size_t)v * co.n_points + i] != 1
-                                           : !dropout_decision(kp.dropout, kp.dropout_seed, (uint32_t)(kp.batch_slot + v), (uint32_t)i);
+                if (keep && !co.keep_dropped) keep = !point_dropped(kp, v, pts.n, i);
                 const unsigned vote = __ballot_sync(0xffffffffu, keep);
                 if (vote)
                 {
@@ -298,20 +329,31 @@ __device__ __forceinline__ void splat_record(float* rec, float* weight, const fl
 // instead of the positions, and does not project; with the radius rule in use the id word also says how many layers it left.
 struct CandIn
 {
-    const float4* rec;   // this view's records
-    const int* count;    // this view's per-block counts
+    const float4* rec;   // the first view's records
+    const int* count;    // the first view's per-block counts, kVisibleSegments per view
+    size_t view_stride;  // records per view
     int seg_cap;
     int parts;           // blocks that share a segment
+};
+// Distances from view to view of a launch that serves several consecutive views (blockIdx.y; the layer planes of a batch
+// follow each other anyway).
+struct ViewStrides
+{
+    size_t accum_floats;
+    size_t list_ints;
 };
 template <int L, int C, bool PLAIN, bool CAND, bool EMIT>
 __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSchedule sched, CandIn cs, const float* __restrict__ texture,
                                                    const float* __restrict__ texture_interleaved, int num_texels,
                                                    const ViewCam* __restrict__ camp, KernelParams kp, LayerTable lt, TileTable tt,
-                                                   float* __restrict__ accum, VisibleList vl, unsigned char* __restrict__ touched_points,
-                                                   unsigned char* __restrict__ touched_texels)
+                                                   float* __restrict__ accum, VisibleList vl, ViewStrides vs,
+                                                   unsigned char* __restrict__ touched_points, unsigned char* __restrict__ touched_texels)
 {
     static_assert(!CAND || PLAIN, "one instantiation reads the streams of both kinds of prepass");
-    const ViewCam& cam = *camp;
+    const int view = (int)blockIdx.y;
+    const ViewCam& cam = camp[view];
+    accum += view * vs.accum_floats;
+    if (EMIT) vl = list_of_view(vl, vs.list_ints, view);
     const bool cand_layers = CAND && kp.drop_out_points_by_radius != 0;
     const bool use_normal = PLAIN ? false : kp.check_normal != 0;
     const bool use_radius = PLAIN ? false : kp.drop_out_points_by_radius != 0;
@@ -337,7 +379,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSche
             if (CAND && l >= n_layers) live = false;
             int px = round_half_even_bounded(x), py = round_half_even_bounded(y);
             in[l] = live && (unsigned)px < (unsigned)lt.w[l] && (unsigned)py < (unsigned)lt.h[l];
-            lin[l] = py * lt.w[l] + px;
+            lin[l] = (view * lt.h[l] + py) * lt.w[l] + px;  // 32 bits hold the planes of a group of four views, checked by the entry point
         }
         unsigned pass = 0;  // the depth reads of all layers go out together
 #pragma unroll
@@ -361,7 +403,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSche
     auto make_entry = [&](int i, float4 cur, int n_layers) -> int4
     {
         // the candidate streams hold dropped points only where the list wants them
-        const bool dropped = (!CAND || (EMIT && kp.ghost_gradients)) && point_dropped(kp, i);
+        const bool dropped = (!CAND || (EMIT && kp.ghost_gradients)) && point_dropped(kp, view, pts.n, i);
         if (dropped && !(EMIT && kp.ghost_gradients)) return make_int4(0, 0, 0, 0);
         float x, y;
         unsigned masks;
@@ -400,7 +442,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSche
                 if (code & (1u << l))
                 {
                     const int lin = round_half_even_bounded(y) * lt.w[l] + round_half_even_bounded(x);
-                    splat_record<C>(accum + ((size_t)lt.rec_off[l] + lin) * RS, lt.weight[l] + lin, t);
+                    splat_record<C>(accum + ((size_t)lt.rec_off[l] + lin) * RS, lt.weight[l] + (unsigned)(view * lt.h[l]) * (unsigned)lt.w[l] + lin, t);
                 }
         }
         if (EMIT)
@@ -459,9 +501,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSche
     if (CAND)
     {
         const int segment = (int)blockIdx.x / cs.parts, part = (int)blockIdx.x - segment * cs.parts;
-        const int total = __ldg(cs.count + segment);
+        const int total = __ldg(cs.count + view * kVisibleSegments + segment);
         const int first = (int)((long long)total * part / cs.parts), cnt = (int)((long long)total * (part + 1) / cs.parts);
-        const float4* rec = cs.rec + (size_t)segment * cs.seg_cap;
+        const float4* rec = cs.rec + view * cs.view_stride + (size_t)segment * cs.seg_cap;
         for (int k0 = first; k0 < cnt; k0 += kBlock)
         {
             const int k = k0 + threadIdx.x;
@@ -498,7 +540,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_blend(PointStreams pts, ChunkSche
 // them off 32 at a time with all lanes busy (measured on the 1080p pyramid with 15 % holes: 55 -> 28 us without the
 // environment map, which is what the parked version aims at).
 template <int C>
-__device__ __forceinline__ void resolve_environment_pixel(const LayerTable& lt, const ViewCam& cam, const KernelParams& kp, unsigned r,
+__device__ __forceinline__ void resolve_environment_pixel(const LayerTable& lt, int view, const ViewCam& cam, const KernelParams& kp, unsigned r,
                                                           const float* __restrict__ background, const float* __restrict__ env,
                                                           int env_h, int env_w)
 {
@@ -511,7 +553,7 @@ __device__ __forceinline__ void resolve_environment_pixel(const LayerTable& lt, 
     V2 uv = env_uv_for_pixel(gx, gy, cam.V, cam.K, cam.dist, crop_l);
     BilinearTap tp = bilinear_taps(uv, env_w, env_h);
     const float one_minus_m = 1.0f - kp.mask_background_value;
-    float* color = lt.color[l] + pix;
+    float* color = lt.color[l] + (size_t)view * C * plane + pix;
 #pragma unroll
     for (int c = 0; c < C; ++c)
     {
@@ -526,11 +568,13 @@ __device__ __forceinline__ void resolve_environment_pixel(const LayerTable& lt, 
 }
 
 template <int C>
-__global__ void __launch_bounds__(kBlock, 6) k_resolve(LayerTable lt, const ViewCam* __restrict__ camp, KernelParams kp, float* __restrict__ accum,
+__global__ void __launch_bounds__(kBlock, 6) k_resolve(LayerTable lt, const ViewCam* __restrict__ camp, KernelParams kp, float* __restrict__ accum, ViewStrides vs,
                                                      const float* __restrict__ background, const float* __restrict__ env,
                                                      int env_h, int env_w)
 {
-    const ViewCam& cam = *camp;
+    const int view = (int)blockIdx.y;
+    const ViewCam& cam = camp[view];
+    accum += view * vs.accum_floats;
     constexpr int RS = AccumLayout<C>::kFloats;
     constexpr bool kSplit = AccumLayout<C>::kSplit;
     __shared__ unsigned s_parked[kBlock / 32][64];
@@ -552,7 +596,8 @@ __global__ void __launch_bounds__(kBlock, 6) k_resolve(LayerTable lt, const View
             float4* rec = reinterpret_cast<float4*>(accum + (size_t)r * RS);
             // split layout: the blend kernel counted into the weight image itself (requested together with the record:
             // a dependent second load costs more than the bytes it could save)
-            const float cou_split = kSplit ? __ldcg(lt.weight[l] + pix) : 0.f;
+            const size_t vpix = view * plane + pix;
+            const float cou_split = kSplit ? __ldcg(lt.weight[l] + vpix) : 0.f;
             float v[RS];
 #pragma unroll
             for (int k = 0; k < RS / 4; ++k)
@@ -561,9 +606,9 @@ __global__ void __launch_bounds__(kBlock, 6) k_resolve(LayerTable lt, const View
                 v[4 * k] = a.x; v[4 * k + 1] = a.y; v[4 * k + 2] = a.z; v[4 * k + 3] = a.w;
             }
             const float cou = kSplit ? cou_split : v[C < RS ? C : 0];
-            float* color = lt.color[l] + pix;
-            if (!kSplit) lt.weight[l][pix] = cou;
-            if (lt.mask[l]) lt.mask[l][pix] = cou == 0.f ? kp.mask_background_value : 1.f;
+            float* color = lt.color[l] + (size_t)view * C * plane + pix;
+            if (!kSplit) lt.weight[l][vpix] = cou;
+            if (lt.mask[l]) lt.mask[l][vpix] = cou == 0.f ? kp.mask_background_value : 1.f;
             if (cou == 0.f)
             {
                 hole = env != nullptr;
@@ -594,23 +639,24 @@ __global__ void __launch_bounds__(kBlock, 6) k_resolve(LayerTable lt, const View
             if (n_parked >= 32)
             {
                 n_parked -= 32;
-                resolve_environment_pixel<C>(lt, cam, kp, parked[n_parked + lane], background, env, env_h, env_w);
+                resolve_environment_pixel<C>(lt, view, cam, kp, parked[n_parked + lane], background, env, env_h, env_w);
             }
             __syncwarp();
         }
     }
-    if (lane < n_parked) resolve_environment_pixel<C>(lt, cam, kp, parked[lane], background, env, env_h, env_w);
+    if (lane < n_parked) resolve_environment_pixel<C>(lt, view, cam, kp, parked[lane], background, env, env_h, env_w);
 }
 
 // ------------------------------------------------------------------------------------------------------
 // What one forward call decided once for all its views.
 struct ForwardPlan
 {
-    float* accum;
+    float* accum;         // blend_views accumulators
+    size_t accum_stride;  // floats from accumulator to accumulator
+    int blend_views;      // views that are blended in one launch
     bool env;
     int32_t* list_base;   // null = no visible list
     int w, h;             // layer-0 size (geometry of the visible list)
-    int num_views;
     char* large;          // large region of a full workspace (candidate streams), null = small workspace
     bool stream_plain;    // candidate streams also for pinhole views without normal test and radius rule
     LargeRegion lr;
@@ -621,9 +667,11 @@ struct ForwardPlan
     unsigned char* touched_texels;
 };
 
+// One group of up to kCandViews consecutive views, `view` the first: depth prepass of all of them, then blend and resolve,
+// plan.blend_views at a time. lt, kp and cams are the first view's.
 template <int L, int C, bool PLAIN>
-static adop_status launch_view_forward_impl(const PointStreams& pts, const adop_scene* s, const ViewCam* cam, const KernelParams& kp,
-                                            const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int depth_views)
+static adop_status launch_group_forward_impl(const PointStreams& pts, const adop_scene* s, const ViewCam* cams, const KernelParams& kp,
+                                             const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int views)
 {
     static const int g_depth = resident_grid(k_depth_prepass<L, PLAIN, 4, false>, 1ll << 40);
     static const int g_depth_cand = resident_grid(k_depth_prepass<L, PLAIN, 4, true>, 1ll << 40);
@@ -660,106 +708,116 @@ static adop_status launch_view_forward_impl(const PointStreams& pts, const adop_
     co.view_stride = plan.cand_view_stride;
     co.seg_cap = seg_cap;
     co.keep_dropped = emit && kp.ghost_gradients;
-    co.n_points = pts.n;
-    // the depth prepass of this view was done by the launch of its group's first view, unless this is that view
-    if (depth_views > 0)
-    {
 #define ADOP_PREPASS(VV)                                                                                                         \
-    if (cand) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, true><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cam, kp, lt, co))); \
-    else ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cam, kp, lt, co)));
-        switch (depth_views)
-        {
-            case 1: ADOP_PREPASS(1) break;
-            case 2: ADOP_PREPASS(2) break;
-            case 3: ADOP_PREPASS(3) break;
-            default: ADOP_PREPASS(4) break;
-        }
+    if (cand) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, true><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cams, kp, lt, co))); \
+    else ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cams, kp, lt, co)));
+    switch (views)
+    {
+        case 1: ADOP_PREPASS(1) break;
+        case 2: ADOP_PREPASS(2) break;
+        case 3: ADOP_PREPASS(3) break;
+        default: ADOP_PREPASS(4) break;
+    }
 #undef ADOP_PREPASS
-        // the second cloud goes into the same depth planes (PointRenderer.cu:1421-1424); never through candidate streams
-        if (plan.outliers.n > 0)
+    // the second cloud goes into the same depth planes (PointRenderer.cu:1421-1424); never through candidate streams
+    const PointStreams& op = plan.outliers;
+    const int oneed = (op.n + kBlock - 1) / kBlock;
+    if (op.n > 0)
+    {
+        const int og = oneed < g_depth ? oneed : g_depth;
+        CandOut none;
+        none.rec = nullptr; none.count = nullptr; none.view_stride = 0; none.seg_cap = 0; none.keep_dropped = 0;
+#define ADOP_PREPASS_OUT(VV) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<og, kBlock, 0, st>>>(op, make_chunk_schedule(op.n, og), cams, kp, lt, none)))
+        switch (views)
         {
-            const PointStreams& op = plan.outliers;
-            const int oneed = (op.n + kBlock - 1) / kBlock;
-            const int og = oneed < g_depth ? oneed : g_depth;
-            CandOut none;
-            none.rec = nullptr; none.count = nullptr; none.view_stride = 0; none.seg_cap = 0; none.keep_dropped = 0; none.n_points = 0;
-#define ADOP_PREPASS_OUT(VV) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<og, kBlock, 0, st>>>(op, make_chunk_schedule(op.n, og), cam, kp, lt, none)))
-            switch (depth_views)
-            {
-                case 1: ADOP_PREPASS_OUT(1); break;
-                case 2: ADOP_PREPASS_OUT(2); break;
-                case 3: ADOP_PREPASS_OUT(3); break;
-                default: ADOP_PREPASS_OUT(4); break;
-            }
-#undef ADOP_PREPASS_OUT
+            case 1: ADOP_PREPASS_OUT(1); break;
+            case 2: ADOP_PREPASS_OUT(2); break;
+            case 3: ADOP_PREPASS_OUT(3); break;
+            default: ADOP_PREPASS_OUT(4); break;
         }
+#undef ADOP_PREPASS_OUT
     }
-    VisibleList vl = make_visible_list(plan.list_base, pts.n, plan.w, plan.h, view);
-    if (vl.header) ADOP_CUDA_TRY(cudaMemsetAsync(vl.header, 0, sizeof(int) * visible_list_clear_ints(plan.w, plan.h, pts.n), st));
-    CandIn ci;
-    ci.rec = cand ? co.rec + (size_t)(view % kCandViews) * plan.cand_view_stride : nullptr;
-    ci.count = cand ? co.count + (view % kCandViews) * kVisibleSegments : nullptr;
-    ci.seg_cap = seg_cap;
-    ci.parts = parts;
-#define ADOP_BLEND(PLAIN_, CAND_, EMIT_)                                                                                                 \
-    ADOP_LAUNCH("k_blend", st, (k_blend<L, C, PLAIN_, CAND_, EMIT_><<<grid_blend, kBlock, 0, st>>>(                               \
-                                   pts, make_chunk_schedule(pts.n, grid_blend), ci, s->texture, s->texture_interleaved, s->num_texels, cam, kp, lt, plan.tiles, plan.accum, vl, emit ? plan.touched_points : nullptr, emit ? plan.touched_texels : nullptr)))
-    if (cand)
-    {
-        if (emit) ADOP_BLEND(true, true, true); else ADOP_BLEND(true, true, false);
-    }
-    else
-    {
-        if (emit) ADOP_BLEND(PLAIN, false, true); else ADOP_BLEND(PLAIN, false, false);
-    }
-    // the second cloud is blended into the same accumulator (PointRenderer.cu:1437-1440), from its positions, without a list
-    if (plan.outliers.n > 0)
-    {
-        const PointStreams& op = plan.outliers;
-        const int oneed = (op.n + kBlock - 1) / kBlock;
-        const int og = oneed < g_blend ? oneed : g_blend;
-        CandIn no_cand;
-        no_cand.rec = nullptr; no_cand.count = nullptr; no_cand.seg_cap = 0; no_cand.parts = 1;
-        VisibleList no_list = make_visible_list(nullptr, op.n, plan.w, plan.h, view);
-        ADOP_LAUNCH("k_blend", st, (k_blend<L, C, PLAIN, false, false><<<og, kBlock, 0, st>>>(
-                                       op, make_chunk_schedule(op.n, og), no_cand, s->texture, s->texture_interleaved, s->num_texels, cam, kp, lt,
-                                       plan.tiles, plan.accum, no_list, nullptr, nullptr)));
-    }
-#undef ADOP_BLEND
-    unsigned total = lt.rec_off[kMaxLayers];
+    const unsigned total = lt.rec_off[kMaxLayers];
     int grid_px = (int)((total + kBlock - 1) / kBlock);
-    if (grid_px > g_resolve) grid_px = g_resolve;
-    ADOP_LAUNCH("k_resolve", st, (k_resolve<C><<<grid_px, kBlock, 0, st>>>(lt, cam, kp, plan.accum, s->background,
-                                                                          plan.env ? s->env_map : nullptr, s->env_h, s->env_w)));
+    ViewStrides vs;
+    vs.accum_floats = plan.accum_stride;
+    vs.list_ints = plan.list_base ? visible_list_ints(pts.n, plan.w, plan.h) : 0;
+    for (int v = 0; v < views; v += plan.blend_views)
+    {
+        const unsigned n_views = (unsigned)(views - v < plan.blend_views ? views - v : plan.blend_views);
+        const LayerTable ltv = layer_table_of_view(lt, C, v);
+        KernelParams kv = kp;
+        kv.batch_slot += v;
+        if (kv.dropout_mask) kv.dropout_mask += (size_t)v * pts.n;
+        const VisibleList vl = make_visible_list(plan.list_base, pts.n, plan.w, plan.h, view + v);
+        CandIn ci;
+        ci.rec = cand ? co.rec + (size_t)v * plan.cand_view_stride : nullptr;
+        ci.count = cand ? co.count + v * kVisibleSegments : nullptr;
+        ci.view_stride = plan.cand_view_stride;
+        ci.seg_cap = seg_cap;
+        ci.parts = parts;
+#define ADOP_BLEND(PLAIN_, CAND_, EMIT_)                                                                                         \
+    ADOP_LAUNCH("k_blend", st, (k_blend<L, C, PLAIN_, CAND_, EMIT_><<<dim3((unsigned)grid_blend, n_views), kBlock, 0, st>>>(     \
+                                   pts, make_chunk_schedule(pts.n, grid_blend), ci, s->texture, s->texture_interleaved, s->num_texels, cams + v, kv, ltv, plan.tiles, plan.accum, vl, vs, emit ? plan.touched_points : nullptr, emit ? plan.touched_texels : nullptr)))
+        if (cand)
+        {
+            if (emit) ADOP_BLEND(true, true, true); else ADOP_BLEND(true, true, false);
+        }
+        else
+        {
+            if (emit) ADOP_BLEND(PLAIN, false, true); else ADOP_BLEND(PLAIN, false, false);
+        }
+#undef ADOP_BLEND
+        // the second cloud is blended into the same accumulator (PointRenderer.cu:1437-1440), from its positions, without a list
+        if (op.n > 0)
+        {
+            const int og = oneed < g_blend ? oneed : g_blend;
+            CandIn no_cand;
+            no_cand.rec = nullptr; no_cand.count = nullptr; no_cand.view_stride = 0; no_cand.seg_cap = 0; no_cand.parts = 1;
+            KernelParams ko = kv;  // the mask's rows are as long as the main cloud: one view at a time steps through them by hand
+            const VisibleList no_list = make_visible_list(nullptr, op.n, plan.w, plan.h, view);
+            for (unsigned k = 0; k < n_views; ++k)
+            {
+                ADOP_LAUNCH("k_blend", st, (k_blend<L, C, PLAIN, false, false><<<og, kBlock, 0, st>>>(
+                                               op, make_chunk_schedule(op.n, og), no_cand, s->texture, s->texture_interleaved, s->num_texels, cams + v + k, ko,
+                                               layer_table_of_view(ltv, C, (int)k), plan.tiles, plan.accum + k * plan.accum_stride, no_list, vs, nullptr, nullptr)));
+                ++ko.batch_slot;
+                if (ko.dropout_mask) ko.dropout_mask += pts.n;
+            }
+        }
+        const int per_view = (g_resolve + (int)n_views - 1) / (int)n_views;
+        ADOP_LAUNCH("k_resolve", st, (k_resolve<C><<<dim3((unsigned)(grid_px < per_view ? grid_px : per_view), n_views), kBlock, 0, st>>>(
+                                         ltv, cams + v, kv, plan.accum, vs, s->background, plan.env ? s->env_map : nullptr, s->env_h, s->env_w)));
+    }
     ADOP_CUDA_TRY(cudaGetLastError());
     return ADOP_OK;
 }
 
 template <int L, int C>
-static adop_status launch_view_forward(const PointStreams& pts, const adop_scene* s, const ViewCam* cam, const KernelParams& kp,
-                                       const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int depth_views)
+static adop_status launch_group_forward(const PointStreams& pts, const adop_scene* s, const ViewCam* cams, const KernelParams& kp,
+                                        const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int views)
 {
     // the common case - no normal test (or no normals) and no radius drop-out - gets kernels without that code
     const bool plain = !(kp.check_normal && (pts.normal || plan.outliers.normal)) && !kp.drop_out_points_by_radius;
-    return plain ? launch_view_forward_impl<L, C, true>(pts, s, cam, kp, lt, plan, st, view, depth_views)
-                 : launch_view_forward_impl<L, C, false>(pts, s, cam, kp, lt, plan, st, view, depth_views);
+    return plain ? launch_group_forward_impl<L, C, true>(pts, s, cams, kp, lt, plan, st, view, views)
+                 : launch_group_forward_impl<L, C, false>(pts, s, cams, kp, lt, plan, st, view, views);
 }
 
 template <int C>
-static adop_status dispatch_layers_forward(int L, const PointStreams& pts, const adop_scene* s, const ViewCam* cam,
+static adop_status dispatch_layers_forward(int L, const PointStreams& pts, const adop_scene* s, const ViewCam* cams,
                                            const KernelParams& kp, const LayerTable& lt, const ForwardPlan& plan,
-                                           cudaStream_t st, int view, int depth_views)
+                                           cudaStream_t st, int view, int views)
 {
     switch (L)
     {
-        case 1: return launch_view_forward<1, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 2: return launch_view_forward<2, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 3: return launch_view_forward<3, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 4: return launch_view_forward<4, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 5: return launch_view_forward<5, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 6: return launch_view_forward<6, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 7: return launch_view_forward<7, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
-        case 8: return launch_view_forward<8, C>(pts, s, cam, kp, lt, plan, st, view, depth_views);
+        case 1: return launch_group_forward<1, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 2: return launch_group_forward<2, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 3: return launch_group_forward<3, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 4: return launch_group_forward<4, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 5: return launch_group_forward<5, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 6: return launch_group_forward<6, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 7: return launch_group_forward<7, C>(pts, s, cams, kp, lt, plan, st, view, views);
+        case 8: return launch_group_forward<8, C>(pts, s, cams, kp, lt, plan, st, view, views);
     }
     return ADOP_ERR_INVALID_ARGUMENT;
 }
@@ -790,16 +848,20 @@ extern "C" size_t adop_raster_workspace_bytes_full(int32_t num_points, int32_t n
 {
     const size_t small = adop_raster_workspace_bytes(w, h, layers, channels);
     if (small == 0 || num_points < 0 || num_views <= 0) return 0;
-    // candidate streams of a group of views
-    return workspace_large_offset(w, h, layers, channels) + large_region_layout(num_points, num_views).total;
+    // candidate streams of a group of views, accumulators of a group of small ones
+    LayerTable lt;
+    fill_layer_dims(w, h, layers, &lt);
+    const size_t accum_bytes = (size_t)lt.rec_off[kMaxLayers] * (channels % 4 == 0 ? channels : record_floats(channels)) * sizeof(float);
+    return workspace_large_offset(w, h, layers, channels) + large_region_layout(num_points, num_views, accum_bytes).total;
 }
 
 extern "C" adop_status adop_texture_interleave(const float* texture, float* out, int32_t channels, int32_t num_texels, void* stream)
 {
     if (!texture || !out || channels <= 0 || num_texels <= 0) return ADOP_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int grid = (num_texels + kBlock - 1) / kBlock;
-    if (grid > sm_count() * 16) grid = sm_count() * 16;
+    const long long vectors = (long long)num_texels * (channels == 8 ? 2 : (channels == 16 ? 4 : 1));
+    long long blocks = (vectors + kBlock - 1) / kBlock;
+    const int grid = (int)(blocks > sm_count() * 16 ? sm_count() * 16 : blocks);
     switch (channels)
     {
         case 4: ADOP_LAUNCH("k_texture_interleave", st, (k_texture_interleave<1><<<grid, kBlock, 0, st>>>(texture, out, channels, num_texels))); break;
@@ -816,8 +878,9 @@ extern "C" adop_status adop_texture_deinterleave(const float* in, float* out, in
 {
     if (!in || !out || channels <= 0 || num_texels <= 0) return ADOP_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int grid = (num_texels + kBlock - 1) / kBlock;
-    if (grid > sm_count() * 16) grid = sm_count() * 16;
+    const long long vectors = (long long)num_texels * (channels == 8 ? 2 : (channels == 16 ? 4 : 1));
+    long long blocks = (vectors + kBlock - 1) / kBlock;
+    const int grid = (int)(blocks > sm_count() * 16 ? sm_count() * 16 : blocks);
     switch (channels)
     {
         case 4: ADOP_LAUNCH("k_texture_deinterleave", st, (k_texture_deinterleave<1><<<grid, kBlock, 0, st>>>(in, out, channels, num_texels, accumulate))); break;
@@ -860,23 +923,40 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     LayerTable base;
     fill_layer_dims(w0, h0, L, &base);
     ViewCam* cams = static_cast<ViewCam*>(io->workspace);
-    float* accum = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + kCamRegionBytes);
     const bool split = C % 4 == 0;  // AccumLayout: colour sums only, the counts go into the weight images
-    const size_t accum_bytes = (size_t)base.rec_off[kMaxLayers] * (split ? C : record_floats(C)) * sizeof(float);
-    ADOP_CUDA_TRY(cudaMemsetAsync(accum, 0, accum_bytes, st));
-    if (split)
-        for (int l = 0; l < L; ++l)
-            ADOP_CUDA_TRY(cudaMemsetAsync(io->layers[l].weight, 0, sizeof(float) * (size_t)B * base.w[l] * base.h[l], st));
+    const size_t accum_floats = (size_t)base.rec_off[kMaxLayers] * (split ? C : record_floats(C));
+    // A workspace of adop_raster_workspace_bytes_full has a large region behind the pixel records: candidate streams from
+    // the depth prepass to the blend kernel, and accumulators for a group of views where they are small.
+    float* accum = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + kCamRegionBytes);
+    int accum_views = 1;
+    char* large = nullptr;
+    const LargeRegion lr = large_region_layout(N, B, accum_floats * sizeof(float));
+    if (io->workspace_bytes >= adop_raster_workspace_bytes_full(N, B, w0, h0, L, C))
+    {
+        large = static_cast<char*>(io->workspace) + workspace_large_offset(w0, h0, L, C);
+        if (lr.accum_views > 1)
+        {
+            accum = reinterpret_cast<float*>(large + lr.accum);
+            accum_views = lr.accum_views;
+        }
+    }
     const int sms = sm_count();
-    // depth.fill_(100000), PointRenderer.cu:1045 (weights and colours are written by the resolve kernel)
+    // the accumulator, depth.fill_(100000) (PointRenderer.cu:1045), the counts, the cursors of the visible lists (colours, and
+    // the weights of the other layout, are written by the resolve kernel)
+    unsigned depth_bits;
+    const float depth_init = kDepthInit;
+    memcpy(&depth_bits, &depth_init, sizeof(depth_bits));
+    FillTable fills;
+    fills.add(accum, accum_floats * accum_views, 0u);
     for (int l = 0; l < L; ++l)
     {
-        size_t n = (size_t)B * base.w[l] * base.h[l];
-        if (n == 0) continue;
-        int grid = (int)((n / 4 + kBlock - 1) / kBlock) + 1;
-        if (grid > sms * 16) grid = sms * 16;
-        ADOP_LAUNCH("k_fill", st, (k_fill<<<grid, kBlock, 0, st>>>(io->layers[l].depth, n, kDepthInit)));
+        const size_t n = (size_t)B * base.w[l] * base.h[l];
+        fills.add(io->layers[l].depth, n, depth_bits);
+        if (split) fills.add(io->layers[l].weight, n, 0u);
     }
+    if (io->visible_list) fills.add(io->visible_list, visible_list_clear_ints(w0, h0, N), 0u, (size_t)B, visible_list_ints(N, w0, h0));
+    const adop_status fs = launch_fills(fills, st);
+    if (fs != ADOP_OK) return fs;
     // optional packed depth|index planes: all layers or none
     const bool packed = io->packed_depth[0] != nullptr;
     for (int l = 0; l < L; ++l)
@@ -884,10 +964,7 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
             return ADOP_ERR_INVALID_ARGUMENT;
     if (packed)
     {
-        unsigned init_bits;
-        const float init_depth = kDepthInit;
-        memcpy(&init_bits, &init_depth, sizeof(init_bits));
-        const unsigned long long empty = ((unsigned long long)init_bits << 32) | 0xFFFFFFFFull;
+        const unsigned long long empty = ((unsigned long long)depth_bits << 32) | 0xFFFFFFFFull;
         for (int l = 0; l < L; ++l)
         {
             size_t n = (size_t)B * base.w[l] * base.h[l];
@@ -906,10 +983,11 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     pts.n = N;
     ForwardPlan plan;
     plan.accum = accum;
+    plan.accum_stride = accum_floats;
+    plan.blend_views = accum_views;
     plan.env = env;
     plan.list_base = io->visible_list;
     plan.w = w0; plan.h = h0;
-    plan.num_views = B;
     plan.tiles = make_tile_table(w0, h0, N);
     // flags "the backward pass of these views can touch this chunk": zeroed here, set by the blend kernel where it lists a
     // point; descriptor columns follow the point numbers only without an index array, else every texel chunk counts as touched
@@ -929,21 +1007,18 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     plan.outliers.normal = s->outlier_normal;
     plan.outliers.index = s->outlier_index;
     plan.outliers.n = s->outlier_position ? s->num_outliers : 0;
-    plan.large = nullptr;
+    plan.large = large;
     // Pinhole views, no normal test, no radius rule: the streams cost the prepass the depth reads of the finest layer and the
     // records, and save the blend kernel the hidden points. Per view at 1080p, four layers, four channels, prepass + blend: 4.8
     // points per pixel 196 us without and 205 us with streams, 14.5 points per pixel 455 and 361 us; 4K, six layers, eight
     // channels, 6.0 points per pixel 1515 and 1391 us.
     plan.stream_plain = (double)N >= 5.5 * (double)w0 * (double)h0;
     for (int b = 0; b < B; ++b) plan.stream_plain = plan.stream_plain || views[b].camera_model == ADOP_CAMERA_OCAM;
-    plan.lr = large_region_layout(N, B);
+    plan.lr = lr;
     plan.cand_view_stride = entry_capacity(N);
-    // A workspace of adop_raster_workspace_bytes_full has a large region behind the pixel records: candidate streams from
-    // the depth prepass to the accept kernel, and the accept kernel's entry segments.
-    if (io->workspace_bytes >= adop_raster_workspace_bytes_full(N, B, w0, h0, L, C))
-        plan.large = static_cast<char*>(io->workspace) + workspace_large_offset(w0, h0, L, C);
     // the pose and intrinsics tensors live on the device; the per-view cameras are gathered there, a chunk at a time
-    for (int b = 0; b < B; ++b)
+    static_assert(kCamChunk % kCandViews == 0, "a group of views never straddles a camera chunk");
+    for (int b = 0; b < B; b += kCandViews)
     {
         if (b % kCamChunk == 0)
         {
@@ -951,36 +1026,36 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
             fill_cam_chunk(&src, s, views + b, B - b < kCamChunk ? B - b : kCamChunk);
             ADOP_LAUNCH("k_build_cams", st, (k_build_cams<<<1, kCamChunk, 0, st>>>(src, cams)));
         }
+        const int group = B - b < kCandViews ? B - b : kCandViews;
         LayerTable lt = base;
         for (int l = 0; l < L; ++l)
         {
-            size_t plane = (size_t)base.w[l] * base.h[l];
-            lt.depth[l] = io->layers[l].depth + (size_t)b * plane;
-            lt.weight[l] = io->layers[l].weight + (size_t)b * plane;
-            lt.color[l] = io->layers[l].color + (size_t)b * C * plane;
-            lt.mask[l] = (rp->output_background_mask && io->layers[l].mask) ? io->layers[l].mask + (size_t)b * plane : nullptr;
+            lt.depth[l] = io->layers[l].depth;
+            lt.weight[l] = io->layers[l].weight;
+            lt.color[l] = io->layers[l].color;
+            lt.mask[l] = rp->output_background_mask ? io->layers[l].mask : nullptr;
         }
-        KernelParams kp = make_kernel_params(rp, io->dropout_mask, N, b);
+        lt = layer_table_of_view(lt, C, b);
+        const KernelParams kp = make_kernel_params(rp, io->dropout_mask, N, b);
         const ViewCam* cam = cams + (b % kCamChunk);
         if (packed)
-        {
-            PackedPlanes pp;
-            for (int l = 0; l < kMaxLayers; ++l)
-                pp.plane[l] = l < L ? reinterpret_cast<unsigned long long*>(io->packed_depth[l]) + (size_t)b * base.w[l] * base.h[l] : nullptr;
-            static const int g_packed = resident_grid(k_depth_prepass_packed, 1ll << 40);
-            const int need = (N + kBlock - 1) / kBlock;
-            ADOP_LAUNCH("k_depth_prepass_packed", st, (k_depth_prepass_packed<<<need < g_packed ? (need < 1 ? 1 : need) : g_packed, kBlock, 0, st>>>(
-                                                          pts, cam, kp, lt, pp)));
-        }
-        // depth prepass in groups of four consecutive views (a group never straddles a camera chunk: 64 = 16 x 4)
-        const int depth_views = (b % 4 == 0) ? (B - b < 4 ? B - b : 4) : 0;
+            for (int v = 0; v < group; ++v)
+            {
+                PackedPlanes pp;
+                for (int l = 0; l < kMaxLayers; ++l)
+                    pp.plane[l] = l < L ? reinterpret_cast<unsigned long long*>(io->packed_depth[l]) + (size_t)(b + v) * base.w[l] * base.h[l] : nullptr;
+                static const int g_packed = resident_grid(k_depth_prepass_packed, 1ll << 40);
+                const int need = (N + kBlock - 1) / kBlock;
+                ADOP_LAUNCH("k_depth_prepass_packed", st, (k_depth_prepass_packed<<<need < g_packed ? (need < 1 ? 1 : need) : g_packed, kBlock, 0, st>>>(
+                                                              pts, cam + v, kp, lt, pp)));
+            }
         adop_status r;
         switch (C)
         {
-            case 3: r = dispatch_layers_forward<3>(L, pts, s, cam, kp, lt, plan, st, b, depth_views); break;
-            case 4: r = dispatch_layers_forward<4>(L, pts, s, cam, kp, lt, plan, st, b, depth_views); break;
-            case 8: r = dispatch_layers_forward<8>(L, pts, s, cam, kp, lt, plan, st, b, depth_views); break;
-            case 16: r = dispatch_layers_forward<16>(L, pts, s, cam, kp, lt, plan, st, b, depth_views); break;
+            case 3: r = dispatch_layers_forward<3>(L, pts, s, cam, kp, lt, plan, st, b, group); break;
+            case 4: r = dispatch_layers_forward<4>(L, pts, s, cam, kp, lt, plan, st, b, group); break;
+            case 8: r = dispatch_layers_forward<8>(L, pts, s, cam, kp, lt, plan, st, b, group); break;
+            case 16: r = dispatch_layers_forward<16>(L, pts, s, cam, kp, lt, plan, st, b, group); break;
             default:
                 snprintf(last_error_buffer(), 512, "%d descriptor channels: the kernels are built for 3, 4, 8 and 16", C);
                 return ADOP_ERR_UNSUPPORTED;

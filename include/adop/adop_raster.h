@@ -205,13 +205,14 @@ void adop_render_params_default(adop_render_params* p);
 /* Bytes of scratch that forward/backward need for views of w x h with `layers` layers and `channels`
  * descriptor channels. Replaces the size-keyed PointRendererCache (PointRenderer.h:96-157). */
 size_t adop_raster_workspace_bytes(int32_t w, int32_t h, int32_t layers, int32_t channels);
-/* The same plus 16 bytes per point and view of a group of up to four views (about 64 N bytes): with a workspace of at
- * least this size the depth prepass also hands the projected in-image points of each view to the blend kernel, which then
- * neither reads the cloud again nor projects a second time. Same results either way. Whether it pays depends on the view:
- * measured, the forward pass of a 100 M point cloud through the omnidirectional model gets a third faster (expensive
- * projection, a small part of the cloud in the image), while on 1080p pinhole training views with 70 % of a 10 M point cloud
- * in the image the extra stream costs the prepass more than it saves the blend kernel. The host layers of this library
- * ask for it when a batch has omnidirectional views. */
+/* The same plus 16 bytes per point and view of a group of up to four views (about 64 N bytes) and, where they are small,
+ * accumulators for such a group (48 MB at most). With a workspace of at least this size
+ *   - the depth prepass can hand the projected points that may still be accepted to the blend kernel, which then neither
+ *     reads the cloud again nor projects a second time; the library does so where it pays: omnidirectional views, normal
+ *     test or radius rule in use, or 5.5 points of the cloud per pixel and more;
+ *   - the views of a group of small ones are blended and resolved in one launch each.
+ * Same results either way. The host layers of this library ask for it and fall back to the small workspace where the
+ * device has no room. */
 size_t adop_raster_workspace_bytes_full(int32_t num_points, int32_t num_views, int32_t w, int32_t h, int32_t layers,
                                         int32_t channels);
 
