@@ -15,6 +15,10 @@
 //    are reduced warp -> block in shared memory and leave as one atomic per component and block;
 //  * the all-points kernels read the ghost stencil from one interleaved record per pixel [I_0..I_C-1, G_0..G_C-1] that a
 //    preparation pass builds (a neighbour then costs one or two 32-byte sectors instead of 2C).
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace adop {
@@ -27,10 +31,24 @@ namespace adop {
 //  * with the fused composite, scatters the environment-map gradient (bilinear, 4 taps).
 __host__ __device__ inline int backward_record_floats(int C) { return (2 * C + 3) & ~3; }
 
+// Planes of view `view` of a launch that serves several views: the layer table points at the first of them, the planes of a
+// batch follow each other.
+__device__ __forceinline__ const float* view_weight(const LayerTable& lt, int l, int view) { return lt.weight[l] + (size_t)view * lt.w[l] * lt.h[l]; }
+template <int C>
+__device__ __forceinline__ const float* view_color(const LayerTable& lt, int l, int view) { return lt.color[l] + (size_t)view * C * lt.w[l] * lt.h[l]; }
+template <int C>
+__device__ __forceinline__ const float* view_grad(const LayerTable& lt, int l, int view) { return lt.grad[l] + (size_t)view * C * lt.w[l] * lt.h[l]; }
+// The visible lists of the launch's views: the first one's, and the distance from list to list
+struct ViewLists
+{
+    VisibleList first;
+    size_t view_ints;
+};
+
 // The environment-map gradient of an uncovered pixel (bilinear scatter, 4 taps): as in the forward resolve kernel the
 // uncovered pixels are scattered single-pixel holes, so each warp parks them and works them off 32 at a time.
 template <int C>
-__device__ __forceinline__ void scatter_environment_gradient(const LayerTable& lt, const ViewCam& cam, const KernelParams& kp, unsigned r,
+__device__ __forceinline__ void scatter_environment_gradient(const LayerTable& lt, int view, const ViewCam& cam, const KernelParams& kp, unsigned r,
                                                              float* __restrict__ grad_env, int env_h, int env_w, bool interleaved)
 {
     const int l = layer_of_record(lt, r);
@@ -40,7 +58,7 @@ __device__ __forceinline__ void scatter_environment_gradient(const LayerTable& l
     const int gy = pix / w, gx = pix - gy * w;
     float gup[C];
 #pragma unroll
-    for (int c = 0; c < C; ++c) gup[c] = __ldg(lt.grad[l] + c * plane + pix);
+    for (int c = 0; c < C; ++c) gup[c] = __ldg(view_grad<C>(lt, l, view) + c * plane + pix);
     Intr5 crop_l = scale_intr(cam.crop, __int_as_float((127 - l) << 23));
     V2 uv = env_uv_for_pixel(gx, gy, cam.V, cam.K, cam.dist, crop_l);
     BilinearTap tp = bilinear_taps(uv, env_w, env_h);
@@ -76,16 +94,22 @@ __device__ __forceinline__ void scatter_environment_gradient(const LayerTable& l
     }
 }
 
+struct HoleArgs
+{
+    float* grad_background;
+    float* grad_env;
+    int env_h, env_w;
+    bool env_interleaved;
+};
 template <int C>
-__global__ void __launch_bounds__(kBlock) k_prepare_backward(LayerTable lt, const ViewCam* __restrict__ camp, KernelParams kp,
-                                                              const float* __restrict__ background, float* __restrict__ records,
-                                                              float* __restrict__ grad_background,
-                                                              float* __restrict__ grad_env, int env_h, int env_w, bool env_interleaved,
-                                                              const int* __restrict__ skip_if_nonzero)
+__device__ __forceinline__ void prepare_backward_part(const LayerTable& lt, int view, const ViewCam& cam, const KernelParams& kp,
+                                                      const float* __restrict__ background, float* __restrict__ records, const HoleArgs& ha)
 {
     constexpr int RB = (2 * C + 3) & ~3;
-    if (skip_if_nonzero && __ldg(skip_if_nonzero) != 0) return;  // this pass runs on the visible list: nothing to prepare
-    const ViewCam& cam = *camp;
+    float* __restrict__ grad_background = ha.grad_background;
+    float* __restrict__ grad_env = ha.grad_env;
+    const int env_h = ha.env_h, env_w = ha.env_w;
+    const bool env_interleaved = ha.env_interleaved;
     __shared__ float s_bg[C];
     __shared__ unsigned s_parked[kBlock / 32][64];
     unsigned* parked = s_parked[threadIdx.x >> 5];
@@ -109,13 +133,13 @@ __global__ void __launch_bounds__(kBlock) k_prepare_backward(LayerTable lt, cons
             const unsigned pix = r - lt.rec_off[l];
             const size_t plane = (size_t)lt.w[l] * lt.h[l];
             // every load of the pixel is requested before the coverage is known
-            const float wgt = __ldg(lt.weight[l] + pix);
+            const float wgt = __ldg(view_weight(lt, l, view) + pix);
             float rec[RB];
 #pragma unroll
             for (int c = 0; c < C; ++c)
             {
-                rec[C + c] = __ldcs(lt.grad[l] + c * plane + pix);
-                rec[c] = __ldg(lt.color[l] + c * plane + pix);
+                rec[C + c] = __ldcs(view_grad<C>(lt, l, view) + c * plane + pix);
+                rec[c] = __ldg(view_color<C>(lt, l, view) + c * plane + pix);
             }
             const bool covered = wgt != 0.f;
             if (!covered)
@@ -145,12 +169,12 @@ __global__ void __launch_bounds__(kBlock) k_prepare_backward(LayerTable lt, cons
             if (n_parked >= 32)
             {
                 n_parked -= 32;
-                scatter_environment_gradient<C>(lt, cam, kp, parked[n_parked + lane], grad_env, env_h, env_w, env_interleaved);
+                scatter_environment_gradient<C>(lt, view, cam, kp, parked[n_parked + lane], grad_env, env_h, env_w, env_interleaved);
             }
             __syncwarp();
         }
     }
-    if (lane < n_parked) scatter_environment_gradient<C>(lt, cam, kp, parked[lane], grad_env, env_h, env_w, env_interleaved);
+    if (lane < n_parked) scatter_environment_gradient<C>(lt, view, cam, kp, parked[lane], grad_env, env_h, env_w, env_interleaved);
     if (grad_background)
     {
 #pragma unroll
@@ -162,6 +186,12 @@ __global__ void __launch_bounds__(kBlock) k_prepare_backward(LayerTable lt, cons
         __syncthreads();
         if (threadIdx.x < C && s_bg[threadIdx.x] != 0.f) atomicAdd(grad_background + threadIdx.x, s_bg[threadIdx.x]);
     }
+}
+template <int C>
+__global__ void __launch_bounds__(kBlock) k_prepare_backward(LayerTable lt, const ViewCam* __restrict__ camp, KernelParams kp,
+                                                              const float* __restrict__ background, float* __restrict__ records, HoleArgs ha)
+{
+    prepare_backward_part<C>(lt, 0, *camp, kp, background, records, ha);
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -179,9 +209,10 @@ struct BackwardTargets
     float* count_pose;        // element of this view's image
     float* grad_intrinsics;   // row of this view's camera
     float* count_intrinsics;  // element of this view's camera
-    const float* records;     // interleaved [I | G] per pyramid pixel, written by k_prepare_backward
 };
 
+// interleaved [I | G] of a pyramid pixel, written by the preparation pass (in the same launch where that serves several
+// views: no read-only loads)
 template <int C>
 __device__ __forceinline__ void load_record(const float* records, size_t r, float* out)
 {
@@ -190,7 +221,7 @@ __device__ __forceinline__ void load_record(const float* records, size_t r, floa
 #pragma unroll
     for (int k = 0; k < RB / 4; ++k)
     {
-        float4 a = __ldg(src + k);
+        float4 a = src[k];
         out[4 * k] = a.x; out[4 * k + 1] = a.y; out[4 * k + 2] = a.z; out[4 * k + 3] = a.w;
     }
 }
@@ -306,9 +337,10 @@ __device__ __forceinline__ void geo_shared_init(GeoShared<MODEL>* s)
     if (threadIdx.x < GeoAccum<MODEL>::NI) s->intr[threadIdx.x] = 0.f;
     if (threadIdx.x == 0) { s->cnt = 0.f; s->any = 0; }
 }
-// every thread of the block must call this
+// every thread of the block must call this; image, camera: the view's rows of the tensors, counted from bt's pointers
 template <int MODEL>
-__device__ __forceinline__ void geo_block_reduce(GeoShared<MODEL>* s, const GeoAccum<MODEL>& acc, const BackwardTargets& bt)
+__device__ __forceinline__ void geo_block_reduce(GeoShared<MODEL>* s, const GeoAccum<MODEL>& acc, const BackwardTargets& bt, int image = 0, int camera = 0,
+                                                 int intrinsics_cols = 0)
 {
     constexpr int NI = GeoAccum<MODEL>::NI;
     if (!(bt.grad_pose || bt.grad_intrinsics)) return;
@@ -341,32 +373,24 @@ __device__ __forceinline__ void geo_block_reduce(GeoShared<MODEL>* s, const GeoA
     if (!s->any) return;
     if (bt.grad_pose)
     {
-        if (threadIdx.x < 6) atomicAdd(bt.grad_pose + threadIdx.x, s->pose[threadIdx.x]);
-        if (threadIdx.x == 6) atomicAdd(bt.count_pose, s->cnt);
+        if (threadIdx.x < 6) atomicAdd(bt.grad_pose + (size_t)image * 6 + threadIdx.x, s->pose[threadIdx.x]);
+        if (threadIdx.x == 6) atomicAdd(bt.count_pose + image, s->cnt);
     }
     if (bt.grad_intrinsics)
     {
-        if (threadIdx.x >= 32 && threadIdx.x < 32 + NI) atomicAdd(bt.grad_intrinsics + (threadIdx.x - 32), s->intr[threadIdx.x - 32]);
+        if (threadIdx.x >= 32 && threadIdx.x < 32 + NI) atomicAdd(bt.grad_intrinsics + (size_t)camera * intrinsics_cols + (threadIdx.x - 32), s->intr[threadIdx.x - 32]);
         // the reference counts 1/1024 per pinhole contribution and 1 per OCam contribution (:680-681, :718)
-        if (threadIdx.x == 64) atomicAdd(bt.count_intrinsics, MODEL == kPinholeDistortion ? s->cnt * (1.f / 1024.f) : s->cnt);
+        if (threadIdx.x == 64) atomicAdd(bt.count_intrinsics + camera, MODEL == kPinholeDistortion ? s->cnt * (1.f / 1024.f) : s->cnt);
     }
 }
 
 // K5 (all points): the reference's structure, one thread per point walking its layers (RenderBackward, :396-724). Used
 // when the forward pass recorded no visible list (or a tile's bucket overflowed, or the list was used before).
 template <int C, int MODEL>
-__global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts, const ViewCam* __restrict__ camp, KernelParams kp, LayerTable lt,
-                                                                BackwardTargets bt, int* __restrict__ list_header, int mark_consumed)
+__device__ __forceinline__ void splat_backward_part(const PointStreams& pts, const ViewCam& cam, const KernelParams& kp, const LayerTable& lt, int view,
+                                                    const BackwardTargets& bt, const float* records, int image, int camera, int intrinsics_cols)
 {
     constexpr int RB = (2 * C + 3) & ~3;
-    // Behind a visible list (last kernel of the pass): if the pass ran on the list there is nothing left to do but to mark
-    // the list consumed when its entries were turned into work items.
-    if (list_header && __ldg(list_header + kListGo) != 0)
-    {
-        if (mark_consumed && blockIdx.x == 0 && threadIdx.x == 0) list_header[kListConsumed] = 1;
-        return;
-    }
-    const ViewCam& cam = *camp;
     __shared__ GeoShared<MODEL> s_geo;
     geo_shared_init(&s_geo);
     __syncthreads();
@@ -376,7 +400,7 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pts.n; i += stride)
     {
-        const bool drop_out = point_dropped(kp, 0, pts.n, i);
+        const bool drop_out = point_dropped(kp, view, pts.n, i);
         FetchedPoint f = fetch_point(pts, i);
         RasterPoint q;
         if (!project_for_raster(cam, f.p, f.r, f.n, f.has_normal, kp.check_normal != 0, kp.dist_cutoff, &q,
@@ -397,8 +421,8 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
             const int w = lt.w[l], h = lt.h[l];
             if ((unsigned)px >= (unsigned)w || (unsigned)py >= (unsigned)h) continue;
             const size_t pix = (size_t)py * w + px;
-            const float* __restrict__ D = lt.depth[l];
-            const float* __restrict__ W = lt.weight[l];
+            const float* D = lt.depth[l] + (size_t)view * w * h;
+            const float* W = view_weight(lt, l, view);
             if (q.z > __ldg(D + pix) * kp.depth_accept_plus_one) break;
             const float wgt = __ldg(W + pix);
             const size_t rbase = (size_t)lt.rec_off[l] + pix;
@@ -408,7 +432,7 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
                 if (bt.grad_texture)
                 {
                     float rc[RB];
-                    load_record<C>(bt.records, rbase, rc);
+                    load_record<C>(records, rbase, rc);
                     const float iw = 1.f / wgt;
 #pragma unroll
                     for (int c = 0; c < C; ++c) dg[c] += iw * rc[C + c];
@@ -426,7 +450,7 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
             const size_t nb[4] = {pix - 1, pix + 1, pix - (size_t)w, pix + (size_t)w};
             float rn[4][RB];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) load_record<C>(bt.records, (size_t)lt.rec_off[l] + nb[k], rn[k]);
+            for (int k = 0; k < 4; ++k) load_record<C>(records, (size_t)lt.rec_off[l] + nb[k], rn[k]);
             V2 g = stencil_gradient<C>(kp, T_p, rn, q.z, W, D, nb);
             chain_gradient<MODEL>(cam, kp, f, g, scale, gp, acc);
         }
@@ -437,7 +461,38 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
         }
         if (gp[3] > 0.f && bt.grad_points) atomicAdd(bt.grad_points + i, make_float4(gp[0], gp[1], gp[2], gp[3]));
     }
-    geo_block_reduce<MODEL>(&s_geo, acc, bt);
+    geo_block_reduce<MODEL>(&s_geo, acc, bt, image, camera, intrinsics_cols);
+}
+template <int C, int MODEL>
+__global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts, const ViewCam* __restrict__ camp, const ViewRows* __restrict__ rows,
+                                                                KernelParams kp, LayerTable lt, BackwardTargets bt, const float* records, int intrinsics_cols)
+{
+    splat_backward_part<C, MODEL>(pts, *camp, kp, lt, 0, bt, records, rows->image, rows->camera, intrinsics_cols);
+}
+
+// Behind the visible lists: the last kernel of the pass, one cooperative launch for all its views. A view that ran on its list
+// only has the list marked as consumed when its entries were turned into work items; a view whose list was not usable gets
+// the two all-points steps here. Nearly always there is nothing to do, and a launch per view and step for nothing was
+// 32 of the 130 launches of a 16-view training step.
+template <int C, int MODEL>
+__global__ void __launch_bounds__(kBlock) k_behind_lists(PointStreams pts, const ViewCam* __restrict__ cams, const ViewRows* __restrict__ rows, KernelParams kp,
+                                                          LayerTable lt, BackwardTargets bt, float* records, int intrinsics_cols, ViewLists lists, HoleArgs ha,
+                                                          int views, int mark_consumed)
+{
+    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    for (int view = 0; view < views; ++view)
+    {
+        int* header = list_of_view(lists.first, lists.view_ints, view).header;
+        if (__ldg(header + kListGo) != 0)  // the same in every block: written by an earlier kernel
+        {
+            if (mark_consumed && blockIdx.x == 0 && threadIdx.x == 0) header[kListConsumed] = 1;
+            continue;
+        }
+        prepare_backward_part<C>(lt, view, cams[view], kp, bt.background, records, ha);
+        grid.sync();
+        splat_backward_part<C, MODEL>(pts, cams[view], kp, lt, view, bt, records, rows[view].image, rows[view].camera, intrinsics_cols);
+        grid.sync();  // the next view rewrites the records
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -491,15 +546,17 @@ __device__ __forceinline__ void async_copy_wait_all() { asm volatile("cp.async.w
 
 // Copies layer LAYER's region of the 2C + 1 planes into shared memory (asynchronously; the caller waits).
 template <int C, int LAYER, int STRIDE>
-__device__ __forceinline__ void stage_region(const LayerTable& lt, float* s_tile, int x0, int y0)
+__device__ __forceinline__ void stage_region(const LayerTable& lt, int view, float* s_tile, int x0, int y0)
 {
     constexpr int pitch = region_pitch(LAYER), rows = region_rows(LAYER);
     const int w = lt.w[LAYER], h = lt.h[LAYER];
     const size_t plane = (size_t)w * h;
+    const float* weight = view_weight(lt, LAYER, view);
+    const float* color = view_color<C>(lt, LAYER, view);
+    const float* grad = view_grad<C>(lt, LAYER, view);
     const int sx = LAYER == 0 ? x0 - 4 : (((x0 >> LAYER) - 1) & ~3), sy = (y0 >> LAYER) - 1;
     float* dst = s_tile + region_offset(LAYER);
-    const bool vec = (w & 3) == 0 && ((reinterpret_cast<uintptr_t>(lt.weight[LAYER]) | reinterpret_cast<uintptr_t>(lt.color[LAYER]) |
-                                       reinterpret_cast<uintptr_t>(lt.grad[LAYER])) & 15) == 0;
+    const bool vec = (w & 3) == 0 && ((reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(color) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
     if (vec)
     {
         constexpr int p4 = pitch / 4, per_plane = rows * p4;
@@ -510,7 +567,7 @@ __device__ __forceinline__ void stage_region(const LayerTable& lt, float* s_tile
             const int gy = sy + row, gx = sx + 4 * c4;
             if ((unsigned)gy < (unsigned)h && (unsigned)gx < (unsigned)w)
             {
-                const float* src = p == 0 ? lt.weight[LAYER] : (p <= C ? lt.color[LAYER] + (size_t)(p - 1) * plane : lt.grad[LAYER] + (size_t)(p - 1 - C) * plane);
+                const float* src = p == 0 ? weight : (p <= C ? color + (size_t)(p - 1) * plane : grad + (size_t)(p - 1 - C) * plane);
                 async_copy_16(dst + p * STRIDE + row * pitch + 4 * c4, src + (size_t)gy * w + gx);
             }
         }
@@ -525,17 +582,17 @@ __device__ __forceinline__ void stage_region(const LayerTable& lt, float* s_tile
             const int gy = sy + row, gx = sx + col;
             if ((unsigned)gy < (unsigned)h && (unsigned)gx < (unsigned)w)
             {
-                const float* src = p == 0 ? lt.weight[LAYER] : (p <= C ? lt.color[LAYER] + (size_t)(p - 1) * plane : lt.grad[LAYER] + (size_t)(p - 1 - C) * plane);
+                const float* src = p == 0 ? weight : (p <= C ? color + (size_t)(p - 1) * plane : grad + (size_t)(p - 1 - C) * plane);
                 async_copy_4(dst + p * STRIDE + row * pitch + col, src + (size_t)gy * w + gx);
             }
         }
     }
 }
 template <int C, int LAYER, int STRIDE, int LMAX>
-__device__ __forceinline__ void stage_regions(const LayerTable& lt, float* s_tile, int x0, int y0)
+__device__ __forceinline__ void stage_regions(const LayerTable& lt, int view, float* s_tile, int x0, int y0)
 {
-    if (LAYER < lt.L) stage_region<C, LAYER, STRIDE>(lt, s_tile, x0, y0);
-    if constexpr (LAYER + 1 < LMAX) stage_regions<C, LAYER + 1, STRIDE, LMAX>(lt, s_tile, x0, y0);
+    if (LAYER < lt.L) stage_region<C, LAYER, STRIDE>(lt, view, s_tile, x0, y0);
+    if constexpr (LAYER + 1 < LMAX) stage_regions<C, LAYER + 1, STRIDE, LMAX>(lt, view, s_tile, x0, y0);
 }
 
 // One (point, layer) visit of the backward pass: descriptor gradient and ghost-geometry image gradient of the point's pixel
@@ -592,7 +649,7 @@ struct PointVisit
 };
 // the visit of layer LAYER (and, recursively, of the coarser ones); x, y = the position on this layer, scale = 0.5^LAYER
 template <int C, int LAYER, int STRIDE, int LMAX>
-__device__ __forceinline__ void visit_layers(const LayerTable& lt, const float* s_tile, int x0, int y0, float x, float y, float scale, PointVisit<C>& pv)
+__device__ __forceinline__ void visit_layers(const LayerTable& lt, int view, const float* s_tile, int x0, int y0, float x, float y, float scale, PointVisit<C>& pv)
 {
     if (LAYER < lt.L && (pv.bmask >> LAYER) != 0)  // no coarser layer to visit either: stop
     {
@@ -616,9 +673,9 @@ __device__ __forceinline__ void visit_layers(const LayerTable& lt, const float* 
             {
                 const size_t plane = (size_t)w * h;
                 const size_t pix = (size_t)py * w + px;
-                const float* W = lt.weight[LAYER];
-                const float* I = lt.color[LAYER];
-                const float* G = lt.grad[LAYER];
+                const float* W = view_weight(lt, LAYER, view);
+                const float* I = view_color<C>(lt, LAYER, view);
+                const float* G = view_grad<C>(lt, LAYER, view);
                 visit_layer<C>([&](int p, int dx, int dy) {
                                    const size_t a = pix + dy * w + dx;
                                    return p == 0 ? __ldg(W + a) : (p <= C ? __ldg(I + (size_t)(p - 1) * plane + a) : __ldg(G + (size_t)(p - 1 - C) * plane + a));
@@ -626,15 +683,18 @@ __device__ __forceinline__ void visit_layers(const LayerTable& lt, const float* 
                                pv.drop_out, pv.want_dg, stencil, pv.T_p, pv.bgc, scale, pv.dg, &pv.have_dg, &pv.gx, &pv.gy, &pv.cnt);
             }
         }
-        if constexpr (LAYER + 1 < LMAX) visit_layers<C, LAYER + 1, STRIDE, LMAX>(lt, s_tile, x0, y0, x * 0.5f, y * 0.5f, scale * 0.5f, pv);
+        if constexpr (LAYER + 1 < LMAX) visit_layers<C, LAYER + 1, STRIDE, LMAX>(lt, view, s_tile, x0, y0, x * 0.5f, y * 0.5f, scale * 0.5f, pv);
     }
 }
 
 template <int C, bool DEEP>
 __global__ void __launch_bounds__(kTileThreads, C <= 4 ? (DEEP ? 3 : 4) : (C <= 8 ? 2 : 1))
-    k_backward_tiles(PointStreams pts, KernelParams kp, LayerTable lt, TileTable tt, BackwardTargets bt, VisibleList vl, int want_geo)
+    k_backward_tiles(PointStreams pts, KernelParams kp, LayerTable lt, TileTable tt, BackwardTargets bt, ViewLists lists, int want_geo)
 {
-    // first kernel of the pass: decides whether the pass runs on the list and leaves the decision for the kernels behind it
+    // blockIdx.y = view. First kernel of the pass: decides whether the view runs on its list and leaves the decision for
+    // the kernels behind it
+    const int view = (int)blockIdx.y;
+    const VisibleList vl = list_of_view(lists.first, lists.view_ints, view);
     const bool go = (__ldg(vl.header + kListUnusable) | __ldg(vl.header + kListConsumed)) == 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) vl.header[kListGo] = go ? 1 : 0;
     if (!go) return;  // the all-points kernels take over
@@ -662,7 +722,7 @@ __global__ void __launch_bounds__(kTileThreads, C <= 4 ? (DEEP ? 3 : 4) : (C <= 
         {
             const int n_pass = min(n_pts - pass0, kTilePass);
             __syncthreads();  // the previous readers of the staged data are done
-            if (pass0 == 0) stage_regions<C, 0, STRIDE, LMAX>(lt, s_tile, x0, y0);
+            if (pass0 == 0) stage_regions<C, 0, STRIDE, LMAX>(lt, view, s_tile, x0, y0);
             for (int q = threadIdx.x; q < n_pass; q += kTileThreads) async_copy_16(sE + q, ent + pass0 + q);
             if (threadIdx.x < kSortBins) s_hist[threadIdx.x] = 0;
             async_copy_wait_all();
@@ -730,7 +790,7 @@ __global__ void __launch_bounds__(kTileThreads, C <= 4 ? (DEEP ? 3 : 4) : (C <= 
                 for (int c = 0; c < C; ++c) pv.dg[c] = 0.f;
                 pv.have_dg = false;
                 pv.gx = pv.gy = pv.cnt = 0.f;
-                visit_layers<C, 0, STRIDE, LMAX>(lt, s_tile, x0, y0, __int_as_float(e.z), __int_as_float(e.w), 1.f, pv);
+                visit_layers<C, 0, STRIDE, LMAX>(lt, view, s_tile, x0, y0, __int_as_float(e.z), __int_as_float(e.w), 1.f, pv);
                 if (pv.have_dg) add_descriptor_gradient<C>(bt.grad_texture, bt.grad_texture_interleaved, bt.num_texels, ti, pv.dg);
                 // the entry becomes the chain kernel's work item (every entry of this pass has been read into shared memory)
                 if (want_geo)
@@ -746,16 +806,9 @@ __global__ void __launch_bounds__(kTileThreads, C <= 4 ? (DEEP ? 3 : 4) : (C <= 
 // per four pyramid pixels reads the weights; the holes, scattered single pixels, are parked per warp and worked off 32
 // at a time (gradient of each channel; for the environment map the ray through the inverse camera model and the bilinear
 // scatter).
-struct HoleArgs
-{
-    float* grad_background;
-    float* grad_env;
-    int env_h, env_w;
-    bool env_interleaved;
-};
 // part of k_chain_and_holes: `block` of `blocks` thread blocks
 template <int C>
-__device__ __forceinline__ void hole_gradients_part(const LayerTable& lt, const ViewCam* __restrict__ camp, const KernelParams& kp, const HoleArgs& ha,
+__device__ __forceinline__ void hole_gradients_part(const LayerTable& lt, int view, const ViewCam* __restrict__ camp, const KernelParams& kp, const HoleArgs& ha,
                                                     int block, int blocks)
 {
     float* __restrict__ grad_background = ha.grad_background;
@@ -781,9 +834,9 @@ __device__ __forceinline__ void hole_gradients_part(const LayerTable& lt, const 
         if (grad_background)
         {
 #pragma unroll
-            for (int c = 0; c < C; ++c) g[c] += __ldg(lt.grad[l] + c * plane + pix);
+            for (int c = 0; c < C; ++c) g[c] += __ldg(view_grad<C>(lt, l, view) + c * plane + pix);
         }
-        if (grad_env) scatter_environment_gradient<C>(lt, cam, kp, r, grad_env, env_h, env_w, env_interleaved);
+        if (grad_env) scatter_environment_gradient<C>(lt, view, cam, kp, r, grad_env, env_h, env_w, env_interleaved);
     };
     const unsigned total = lt.rec_off[kMaxLayers];
     const unsigned groups = (total + 3) / 4;
@@ -801,7 +854,7 @@ __device__ __forceinline__ void hole_gradients_part(const LayerTable& lt, const 
             if (r < total)
             {
                 const int l = layer_of_record(lt, r);
-                hole[k] = __ldg(lt.weight[l] + (r - lt.rec_off[l])) == 0.f;
+                hole[k] = __ldg(view_weight(lt, l, view) + (r - lt.rec_off[l])) == 0.f;
             }
         }
 #pragma unroll
@@ -936,7 +989,8 @@ __device__ __forceinline__ bool chain_gradient_sum(const ViewCam& cam, const Ker
 
 // part of k_chain_and_holes: `block` of `blocks` thread blocks
 template <int MODEL>
-__device__ __forceinline__ void point_chain_part(const PointStreams& pts, const ViewCam* __restrict__ camp, const KernelParams& kp, const BackwardTargets& bt,
+__device__ __forceinline__ void point_chain_part(const PointStreams& pts, const ViewCam* __restrict__ camp, const ViewRows* __restrict__ rows,
+                                                 int intrinsics_cols, const KernelParams& kp, const BackwardTargets& bt,
                                                  const VisibleList& vl, const TileTable& tt, int block, int blocks)
 {
     __shared__ ViewCam s_cam;
@@ -1038,20 +1092,26 @@ __device__ __forceinline__ void point_chain_part(const PointStreams& pts, const 
         acc.intr[11] = df * (ps.d[6] * 0.1f); acc.intr[12] = df * (ps.d[7] * 0.1f);
         acc.cnt = ps.cnt;
     }
-    geo_block_reduce<MODEL>(&s_geo, acc, bt);
+    geo_block_reduce<MODEL>(&s_geo, acc, bt, __ldg(&rows->image), __ldg(&rows->camera), intrinsics_cols);
 }
 
-// The chain kernel and the hole kernel of one view in one launch: they are independent, the first waits on memory most of
+// The chain kernel and the hole kernel of the launch's views: they are independent, the first waits on memory most of
 // the time and the second on arithmetic, so side by side they take little more than the longer of the two.
-// Blocks [0, chain_blocks) chain the tile kernel's work items, the others walk the uncovered pixels.
+// blockIdx.y = view; blocks x of [0, chain_blocks) chain the tile kernel's work items, the others walk the uncovered pixels.
+// The views of a launch share the camera model; each view's rows of the pose and intrinsics gradients come from the row
+// table that k_build_cams left behind the camera records.
 template <int C, int MODEL>
 __global__ void __launch_bounds__(kBlock, MODEL == kPinholeDistortion ? 4 : 3)
-    k_chain_and_holes(PointStreams pts, const ViewCam* __restrict__ camp, KernelParams kp, LayerTable lt, BackwardTargets bt, VisibleList vl, TileTable tt,
-                      HoleArgs ha, int chain_blocks)
+    k_chain_and_holes(PointStreams pts, const ViewCam* __restrict__ cams, const ViewRows* __restrict__ rows, KernelParams kp, LayerTable lt, BackwardTargets bt,
+                      int intrinsics_cols, ViewLists lists, TileTable tt, HoleArgs ha, int chain_blocks)
 {
+    const int view = (int)blockIdx.y;
+    const VisibleList vl = list_of_view(lists.first, lists.view_ints, view);
     if (__ldg(vl.header + kListGo) == 0) return;  // the all-points kernels do this work
-    if ((int)blockIdx.x < chain_blocks) point_chain_part<MODEL>(pts, camp, kp, bt, vl, tt, (int)blockIdx.x, chain_blocks);
-    else hole_gradients_part<C>(lt, camp, kp, ha, (int)blockIdx.x - chain_blocks, (int)gridDim.x - chain_blocks);
+    if ((int)blockIdx.x < chain_blocks)
+        point_chain_part<MODEL>(pts, cams + view, rows + view, intrinsics_cols, kp, bt, vl, tt, (int)blockIdx.x, chain_blocks);
+    else
+        hole_gradients_part<C>(lt, view, cams + view, kp, ha, (int)blockIdx.x - chain_blocks, (int)gridDim.x - chain_blocks);
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -1060,7 +1120,10 @@ __global__ void k_normalize_points(float4* g, int n)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    // a point without contributions (w = 0) stays as it is: on a large cloud most points, and then whole sectors, are not
+    // written back
     float4 v = g[i];
+    if (v.w == 0.f) return;
     if (v.w > 0.f) { v.x = v.x / v.w; v.y = v.y / v.w; v.z = v.z / v.w; }
     v.w = 0.f;
     g[i] = v;
@@ -1081,98 +1144,96 @@ __global__ void k_normalize_intrinsics(float* g, const float* cnt, int n, int co
 }
 
 // ------------------------------------------------------------------------------------------------------
-template <int C>
-static adop_status launch_view_backward(const PointStreams& pts, const ViewCam* cam, const KernelParams& kp, const LayerTable& lt,
-                                        const TileTable& tt, const BackwardTargets& bt, float* grad_background, float* grad_env, int env_h,
-                                        int env_w, bool env_interleaved, cudaStream_t st, const VisibleList& vl, int model)
+constexpr int kTileWaves = 2, kChainWaves = 1;
+static int blocks_per_view(int resident, int waves, int views, int most)
 {
-    const int need = (pts.n + kBlock - 1) / kBlock;
-    // With a visible list the tile kernels run; the all-points kernels are launched behind them and return at once unless
-    // the list turns out not to be usable (decided on the device by the first kernel, no host round trip). The debug
-    // stencil rule (test_backward_mode 4) needs the point's depth next to its neighbours' and always takes the all-points
-    // kernels.
-    const bool use_list = vl.header && kp.test_backward_mode != 4;
-    int* go = use_list ? vl.header + kListGo : nullptr;
+    int n = (resident * waves + views - 1) / views;
+    if (n > most) n = most;
+    return n < 1 ? 1 : n;
+}
+
+// The list kernels of `views` consecutive views of one camera model. lt, kp, cams, rows and lists are those of the first;
+// bt's pose and intrinsics rows are the tensors' first rows.
+template <int C, int MODEL>
+static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* cams, const ViewRows* rows, const KernelParams& kp, const LayerTable& lt,
+                                        const TileTable& tt, const BackwardTargets& bt, float* records, int intrinsics_cols, const HoleArgs& ha,
+                                        cudaStream_t st, const ViewLists& lists, int views)
+{
     const int want_geo = (bt.grad_points || bt.grad_pose || bt.grad_intrinsics) ? 1 : 0;
-    if (use_list)
+    const size_t smem = tile_smem_bytes(C, lt.L);
+    const bool deep = lt.L > 4;
+    static size_t smem_set[2] = {0, 0};
+    if (smem > smem_set[deep])
     {
-        const size_t smem = tile_smem_bytes(C, lt.L);
-        const bool deep = lt.L > 4;
-        static size_t smem_set[2] = {0, 0};
-        if (smem > smem_set[deep])
-        {
-            if (deep) ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            else ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            smem_set[deep] = smem;
-        }
-        int per_sm = 0;
-        cudaError_t oe = deep ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, true>, kTileThreads, smem)
-                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, false>, kTileThreads, smem);
-        if (oe != cudaSuccess || per_sm < 1) per_sm = 1;
-        const int g_tiles = per_sm * sm_count();
-        const int grid_tiles = tt.n_tiles < g_tiles ? (tt.n_tiles < 1 ? 1 : tt.n_tiles) : g_tiles;
-        if (deep) ADOP_LAUNCH("k_backward_tiles", st, (k_backward_tiles<C, true><<<grid_tiles, kTileThreads, smem, st>>>(pts, kp, lt, tt, bt, vl, want_geo)));
-        else ADOP_LAUNCH("k_backward_tiles", st, (k_backward_tiles<C, false><<<grid_tiles, kTileThreads, smem, st>>>(pts, kp, lt, tt, bt, vl, want_geo)));
-        if (grad_env || grad_background || want_geo)
-        {
-            HoleArgs ha;
-            ha.grad_background = grad_background; ha.grad_env = grad_env; ha.env_h = env_h; ha.env_w = env_w; ha.env_interleaved = env_interleaved;
-            const unsigned groups = (lt.rec_off[kMaxLayers] + 3) / 4;
-            const int hole_need = (grad_env || grad_background) ? (int)((groups + kBlock - 1) / kBlock) : 0;
-            if (model == kPinholeDistortion)
-            {
-                static const int g = resident_grid(k_chain_and_holes<C, kPinholeDistortion>, 1ll << 40);
-                // the chain blocks get five eighths of the resident blocks when both parts have work (measured: between a half
-                // and three quarters the kernel's time is flat, beyond it rises quickly)
-                int chain_blocks = want_geo ? (hole_need ? g * 5 / 8 : g) : 0;
-                if (chain_blocks > tt.n_tiles) chain_blocks = tt.n_tiles;
-                int hole_blocks = g - chain_blocks < hole_need ? g - chain_blocks : hole_need;
-                if (hole_need && hole_blocks < 1) hole_blocks = 1;
-                ADOP_LAUNCH("k_chain_and_holes", st, (k_chain_and_holes<C, kPinholeDistortion><<<chain_blocks + hole_blocks, kBlock, 0, st>>>(
-                                                         pts, cam, kp, lt, bt, vl, tt, ha, chain_blocks)));
-            }
-            else
-            {
-                static const int g = resident_grid(k_chain_and_holes<C, kOcam>, 1ll << 40);
-                int chain_blocks = want_geo ? (hole_need ? g * 5 / 8 : g) : 0;
-                if (chain_blocks > tt.n_tiles) chain_blocks = tt.n_tiles;
-                int hole_blocks = g - chain_blocks < hole_need ? g - chain_blocks : hole_need;
-                if (hole_need && hole_blocks < 1) hole_blocks = 1;
-                ADOP_LAUNCH("k_chain_and_holes", st, (k_chain_and_holes<C, kOcam><<<chain_blocks + hole_blocks, kBlock, 0, st>>>(
-                                                         pts, cam, kp, lt, bt, vl, tt, ha, chain_blocks)));
-            }
-        }
+        if (deep) ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        else ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        smem_set[deep] = smem;
     }
-    // Behind a visible list these two launches are almost always no-ops that only read the list's control word, so they
-    // get one block per SM (an empty launch costs by its block count); without a list they are the backward pass and fill
-    // the GPU.
-    const int fallback_cap = use_list ? sm_count() : (1 << 30);
+    int per_sm = 0;
+    cudaError_t oe = deep ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, true>, kTileThreads, smem)
+                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, false>, kTileThreads, smem);
+    if (oe != cudaSuccess || per_sm < 1) per_sm = 1;
+    // blocks per view: about kTileWaves times as many blocks as are resident, so that the GPU's own block scheduler evens
+    // out crowded and empty tiles, but never more than a view has tiles
+    const dim3 grid_tiles((unsigned)blocks_per_view(per_sm * sm_count(), kTileWaves, views, tt.n_tiles), (unsigned)views);
+    if (deep) ADOP_LAUNCH("k_backward_tiles", st, (k_backward_tiles<C, true><<<grid_tiles, kTileThreads, smem, st>>>(pts, kp, lt, tt, bt, lists, want_geo)));
+    else ADOP_LAUNCH("k_backward_tiles", st, (k_backward_tiles<C, false><<<grid_tiles, kTileThreads, smem, st>>>(pts, kp, lt, tt, bt, lists, want_geo)));
+    static const int g = resident_grid(k_chain_and_holes<C, MODEL>, 1ll << 40);
+    const unsigned groups = (lt.rec_off[kMaxLayers] + 3) / 4;
+    const int hole_need = (ha.grad_env || ha.grad_background) ? (int)((groups + kBlock - 1) / kBlock) : 0;
+    if (hole_need || want_geo)
     {
-        static const int cap = resident_grid(k_prepare_backward<C>, 1ll << 40);
-        unsigned total = lt.rec_off[kMaxLayers];
-        int grid_px = (int)((total + kBlock - 1) / kBlock);
-        if (grid_px > cap) grid_px = cap;
-        if (grid_px > fallback_cap) grid_px = fallback_cap;
-        ADOP_LAUNCH("k_prepare_backward", st, (k_prepare_backward<C><<<grid_px, kBlock, 0, st>>>(
-                                                  lt, cam, kp, bt.background, const_cast<float*>(bt.records), grad_background,
-                                                  grad_env, env_h, env_w, env_interleaved, go)));
+        // the chain blocks get five eighths of the blocks when both parts have work (measured: between a half and three quarters
+        // the kernel's time is flat, beyond it rises quickly)
+        const int per_view = blocks_per_view(g, kChainWaves, views, 1 << 30);
+        int chain_blocks = want_geo ? (hole_need ? per_view * 5 / 8 : per_view) : 0;
+        if (want_geo && chain_blocks < 1) chain_blocks = 1;
+        if (chain_blocks > tt.n_tiles) chain_blocks = tt.n_tiles;
+        int hole_blocks = per_view - chain_blocks < hole_need ? per_view - chain_blocks : hole_need;
+        if (hole_need && hole_blocks < 1) hole_blocks = 1;
+        ADOP_LAUNCH("k_chain_and_holes", st, (k_chain_and_holes<C, MODEL><<<dim3((unsigned)(chain_blocks + hole_blocks), (unsigned)views), kBlock, 0, st>>>(
+                                                 pts, cams, rows, kp, lt, bt, intrinsics_cols, lists, tt, ha, chain_blocks)));
     }
-    int* header = use_list ? vl.header : nullptr;
-    if (model == kPinholeDistortion)
-    {
-        static const int g = resident_grid(k_splat_backward_all<C, kPinholeDistortion>, 1ll << 40);
-        int grid = need < g ? (need < 1 ? 1 : need) : g;
-        if (grid > fallback_cap) grid = fallback_cap;
-        ADOP_LAUNCH("k_splat_backward_all", st, (k_splat_backward_all<C, kPinholeDistortion><<<grid, kBlock, 0, st>>>(pts, cam, kp, lt, bt, header, want_geo)));
-    }
-    else
-    {
-        static const int g = resident_grid(k_splat_backward_all<C, kOcam>, 1ll << 40);
-        int grid = need < g ? (need < 1 ? 1 : need) : g;
-        if (grid > fallback_cap) grid = fallback_cap;
-        ADOP_LAUNCH("k_splat_backward_all", st, (k_splat_backward_all<C, kOcam><<<grid, kBlock, 0, st>>>(pts, cam, kp, lt, bt, header, want_geo)));
-    }
+    // one block per SM: an empty launch costs by its block count, and a cooperative one has to fit beside other work
+    static const int g_behind = std::min(resident_grid(k_behind_lists<C, MODEL>, 1ll << 40), sm_count());
+    PointStreams a_pts = pts; const ViewCam* a_cams = cams; const ViewRows* a_rows = rows; KernelParams a_kp = kp; LayerTable a_lt = lt; BackwardTargets a_bt = bt;
+    ViewLists a_lists = lists; HoleArgs a_ha = ha; int a_geo = want_geo;
+    void* args[] = {&a_pts, &a_cams, &a_rows, &a_kp, &a_lt, &a_bt, &records, &intrinsics_cols, &a_lists, &a_ha, &views, &a_geo};
+    ADOP_LAUNCH("k_behind_lists", st, ADOP_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_behind_lists<C, MODEL>), dim3((unsigned)g_behind), dim3(kBlock), args, 0, st)));
     ADOP_CUDA_TRY(cudaGetLastError());
+    return ADOP_OK;
+}
+
+// The backward pass of one view without a list.
+template <int C, int MODEL>
+static adop_status launch_all_points_backward(const PointStreams& pts, const ViewCam* cam, const ViewRows* rows, const KernelParams& kp, const LayerTable& lt,
+                                              const BackwardTargets& bt, float* records, int intrinsics_cols, const HoleArgs& ha, cudaStream_t st)
+{
+    static const int g_prepare = resident_grid(k_prepare_backward<C>, 1ll << 40);
+    static const int g_splat = resident_grid(k_splat_backward_all<C, MODEL>, 1ll << 40);
+    const int need = (pts.n + kBlock - 1) / kBlock, need_px = (int)((lt.rec_off[kMaxLayers] + kBlock - 1) / kBlock);
+    ADOP_LAUNCH("k_prepare_backward", st, (k_prepare_backward<C><<<need_px < g_prepare ? need_px : g_prepare, kBlock, 0, st>>>(lt, cam, kp, bt.background, records, ha)));
+    ADOP_LAUNCH("k_splat_backward_all", st, (k_splat_backward_all<C, MODEL><<<need < g_splat ? (need < 1 ? 1 : need) : g_splat, kBlock, 0, st>>>(
+                                                pts, cam, rows, kp, lt, bt, records, intrinsics_cols)));
+    ADOP_CUDA_TRY(cudaGetLastError());
+    return ADOP_OK;
+}
+
+// `views` consecutive views of one camera model, with lists or without; the pointers are the first view's.
+template <int C, int MODEL>
+static adop_status launch_views_backward(const PointStreams& pts, const ViewCam* cams, const ViewRows* rows, const KernelParams& kp, const LayerTable& lt,
+                                         const TileTable& tt, const BackwardTargets& bt, float* records, int intrinsics_cols, const HoleArgs& ha,
+                                         cudaStream_t st, const ViewLists& lists, int views)
+{
+    if (lists.first.header) return launch_list_backward<C, MODEL>(pts, cams, rows, kp, lt, tt, bt, records, intrinsics_cols, ha, st, lists, views);
+    for (int v = 0; v < views; ++v)
+    {
+        KernelParams kv = kp;
+        kv.batch_slot += v;
+        if (kv.dropout_mask) kv.dropout_mask += (size_t)v * pts.n;
+        const adop_status r = launch_all_points_backward<C, MODEL>(pts, cams + v, rows + v, kv, layer_table_of_view(lt, C, v), bt, records, intrinsics_cols, ha, st);
+        if (r != ADOP_OK) return r;
+    }
     return ADOP_OK;
 }
 
@@ -1224,29 +1285,27 @@ extern "C" adop_status adop_raster_backward(const adop_scene* s, const adop_view
             if (views[b].camera_model != ADOP_CAMERA_PINHOLE_DISTORTION) return ADOP_ERR_UNSUPPORTED;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!io->accumulate)
-    {
-        if (io->grad_texture && !io->grad_texture_interleaved)
-            ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_texture, 0, sizeof(float) * (size_t)C * T, st));
-        if (io->grad_background) ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_background, 0, sizeof(float) * C, st));
-        if (io->grad_points) ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_points, 0, sizeof(float) * (size_t)N * 4, st));
-        if (io->grad_pose) ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_pose, 0, sizeof(double) * (size_t)s->num_images * 6, st));
-        if (io->count_pose) ADOP_CUDA_TRY(cudaMemsetAsync(io->count_pose, 0, sizeof(float) * s->num_images, st));
-        if (io->grad_intrinsics) ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_intrinsics, 0, sizeof(float) * (size_t)s->num_cameras * cols, st));
-        if (io->count_intrinsics) ADOP_CUDA_TRY(cudaMemsetAsync(io->count_intrinsics, 0, sizeof(float) * s->num_cameras, st));
-        if (io->grad_env_map && s->env_h > 0 && s->env_w > 0)
-            ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_env_map, 0, sizeof(float) * (size_t)C * s->env_h * s->env_w, st));
-    }
-
     // environment-map gradient: summed in an [eh,ew,C] scratch with vector atomics when the caller gave one
     const bool env_inter = env && io->grad_env_map_interleaved && C % 4 == 0 &&
                            (reinterpret_cast<uintptr_t>(io->grad_env_map_interleaved) & 15) == 0;
-    if (env_inter)
-        ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_env_map_interleaved, 0, sizeof(float) * (size_t)C * s->env_h * s->env_w, st));
     // descriptor gradients stay in the [T,C] buffer when there is no [C,T] tensor to move them into
     const bool interleaved_only = !io->grad_texture && io->grad_texture_interleaved;
-    if (io->grad_texture_interleaved && (io->grad_texture || !io->accumulate))
-        ADOP_CUDA_TRY(cudaMemsetAsync(io->grad_texture_interleaved, 0, sizeof(float) * (size_t)C * T, st));
+    FillTable fills;
+    if (!io->accumulate)
+    {
+        if (!io->grad_texture_interleaved) fills.add(io->grad_texture, (size_t)C * T, 0u);
+        fills.add(io->grad_background, (size_t)C, 0u);
+        fills.add(io->grad_points, (size_t)N * 4, 0u);
+        fills.add(io->grad_pose, (size_t)s->num_images * 12, 0u);
+        fills.add(io->count_pose, (size_t)s->num_images, 0u);
+        fills.add(io->grad_intrinsics, (size_t)s->num_cameras * cols, 0u);
+        fills.add(io->count_intrinsics, (size_t)s->num_cameras, 0u);
+        if (s->env_h > 0 && s->env_w > 0 && !env_inter) fills.add(io->grad_env_map, (size_t)C * s->env_h * s->env_w, 0u);
+    }
+    if (env_inter) fills.add(io->grad_env_map_interleaved, (size_t)C * s->env_h * s->env_w, 0u);
+    if (io->grad_texture || !io->accumulate) fills.add(io->grad_texture_interleaved, (size_t)C * T, 0u);
+    const adop_status fs = launch_fills(fills, st);
+    if (fs != ADOP_OK) return fs;
     LayerTable base;
     fill_layer_dims(views[0].w, views[0].h, L, &base);
     const TileTable tiles = make_tile_table(views[0].w, views[0].h, N);
@@ -1256,54 +1315,70 @@ extern "C" adop_status adop_raster_backward(const adop_scene* s, const adop_view
     pts.normal = s->normal;
     pts.index = s->index;
     pts.n = N;
-    for (int b = 0; b < B; ++b)
+    // The debug stencil rule (test_backward_mode 4) needs the point's depth next to its neighbours' and always takes the
+    // all-points kernels.
+    const bool use_list = io->visible_list && rp->test_backward_mode != 4;
+    float* ge = env ? (env_inter ? io->grad_env_map_interleaved : io->grad_env_map) : nullptr;
+    BackwardTargets bt;
+    bt.texture = s->texture;
+    bt.texture_interleaved = s->texture_interleaved;
+    bt.grad_texture_interleaved = io->grad_texture_interleaved;
+    bt.num_texels = T;
+    bt.background = s->background;
+    // the kernels take a non-null grad_texture as "descriptor gradients wanted" and write the [T,C] buffer if there is one
+    bt.grad_texture = interleaved_only ? io->grad_texture_interleaved : io->grad_texture;
+    bt.grad_points = reinterpret_cast<float4*>(io->grad_points);
+    bt.grad_pose = io->grad_pose;
+    bt.count_pose = io->grad_pose ? io->count_pose : nullptr;
+    bt.grad_intrinsics = io->grad_intrinsics;
+    bt.count_intrinsics = io->grad_intrinsics ? io->count_intrinsics : nullptr;
+    float* records = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + kCamRegionBytes);
+    for (int l = 0; l < L; ++l)
     {
-        LayerTable lt = base;
-        for (int l = 0; l < L; ++l)
+        base.depth[l] = io->layers[l].depth;
+        base.weight[l] = io->layers[l].weight;
+        base.color[l] = io->layers[l].color;
+        base.grad[l] = io->grad_color[l];
+    }
+    const ViewRows* rows = view_rows(cams);
+    for (int b0 = 0; b0 < B; b0 += kCamChunk)
+    {
+        const int chunk = B - b0 < kCamChunk ? B - b0 : kCamChunk;
+        CamChunkSource src;
+        fill_cam_chunk(&src, s, views + b0, chunk);
+        ADOP_LAUNCH("k_build_cams", st, (k_build_cams<<<1, kCamChunk, 0, st>>>(src, cams)));
+        HoleArgs ha;
+        ha.grad_background = io->grad_background; ha.grad_env = ge; ha.env_h = s->env_h; ha.env_w = s->env_w; ha.env_interleaved = env_inter;
+        // runs of consecutive views with the same camera model
+        for (int b = b0, e; b < b0 + chunk; b = e)
         {
-            size_t plane = (size_t)base.w[l] * base.h[l];
-            lt.depth[l] = io->layers[l].depth + (size_t)b * plane;
-            lt.weight[l] = io->layers[l].weight + (size_t)b * plane;
-            lt.color[l] = io->layers[l].color + (size_t)b * C * plane;
-            lt.grad[l] = io->grad_color[l] + (size_t)b * C * plane;
+            for (e = b + 1; e < b0 + chunk && views[e].camera_model == views[b].camera_model; ++e) {}
+            ViewLists lists;
+            // the list's layout (tiles, bucket size) follows from the view size and the point count, as in the forward pass
+            lists.first = make_visible_list(use_list ? const_cast<int32_t*>(io->visible_list) : nullptr, N, views[0].w, views[0].h, b);
+            lists.view_ints = visible_list_ints(N, views[0].w, views[0].h);
+            const LayerTable lt = layer_table_of_view(base, C, b);
+            const KernelParams kp = make_kernel_params(rp, io->dropout_mask, N, b);
+            const bool pinhole = views[b].camera_model == kPinholeDistortion;
+            const ViewCam* cam = cams + (b - b0);
+            const ViewRows* row = rows + (b - b0);
+            adop_status r;
+#define ADOP_VIEWS_BACKWARD(CC)                                                                                                                      \
+    r = pinhole ? launch_views_backward<CC, kPinholeDistortion>(pts, cam, row, kp, lt, tiles, bt, records, cols, ha, st, lists, e - b)               \
+                : launch_views_backward<CC, kOcam>(pts, cam, row, kp, lt, tiles, bt, records, cols, ha, st, lists, e - b)
+            switch (C)
+            {
+                case 3: ADOP_VIEWS_BACKWARD(3); break;
+                case 4: ADOP_VIEWS_BACKWARD(4); break;
+                case 8: ADOP_VIEWS_BACKWARD(8); break;
+                case 16: ADOP_VIEWS_BACKWARD(16); break;
+                default:
+                    snprintf(last_error_buffer(), 512, "%d descriptor channels: the kernels are built for 3, 4, 8 and 16", C);
+                    return ADOP_ERR_UNSUPPORTED;
+            }
+#undef ADOP_VIEWS_BACKWARD
+            if (r != ADOP_OK) return r;
         }
-        KernelParams kp = make_kernel_params(rp, io->dropout_mask, N, b);
-        if (b % kCamChunk == 0)
-        {
-            CamChunkSource src;
-            fill_cam_chunk(&src, s, views + b, B - b < kCamChunk ? B - b : kCamChunk);
-            ADOP_LAUNCH("k_build_cams", st, (k_build_cams<<<1, kCamChunk, 0, st>>>(src, cams)));
-        }
-        const ViewCam* cam = cams + (b % kCamChunk);
-        BackwardTargets bt;
-        bt.texture = s->texture;
-        bt.texture_interleaved = s->texture_interleaved;
-        bt.grad_texture_interleaved = io->grad_texture_interleaved;
-        bt.num_texels = T;
-        bt.background = s->background;
-        // the kernels take a non-null grad_texture as "descriptor gradients wanted" and write the [T,C] buffer if there is one
-        bt.grad_texture = interleaved_only ? io->grad_texture_interleaved : io->grad_texture;
-        bt.grad_points = reinterpret_cast<float4*>(io->grad_points);
-        bt.grad_pose = io->grad_pose ? io->grad_pose + (size_t)views[b].image_index * 6 : nullptr;
-        bt.count_pose = io->grad_pose ? io->count_pose + views[b].image_index : nullptr;
-        bt.grad_intrinsics = io->grad_intrinsics ? io->grad_intrinsics + (size_t)views[b].camera_index * cols : nullptr;
-        bt.count_intrinsics = io->grad_intrinsics ? io->count_intrinsics + views[b].camera_index : nullptr;
-        bt.records = reinterpret_cast<const float*>(static_cast<const char*>(io->workspace) + kCamRegionBytes);
-        float* ge = env ? (env_inter ? io->grad_env_map_interleaved : io->grad_env_map) : nullptr;
-        // the list's layout (tiles, bucket size) follows from the view size and the point count, as in the forward pass
-        VisibleList vl = make_visible_list(const_cast<int32_t*>(io->visible_list), N, views[0].w, views[0].h, b);
-        adop_status r;
-        switch (C)
-        {
-            case 3: r = launch_view_backward<3>(pts, cam, kp, lt, tiles, bt, io->grad_background, ge, s->env_h, s->env_w, env_inter, st, vl, views[b].camera_model); break;
-            case 4: r = launch_view_backward<4>(pts, cam, kp, lt, tiles, bt, io->grad_background, ge, s->env_h, s->env_w, env_inter, st, vl, views[b].camera_model); break;
-            case 8: r = launch_view_backward<8>(pts, cam, kp, lt, tiles, bt, io->grad_background, ge, s->env_h, s->env_w, env_inter, st, vl, views[b].camera_model); break;
-            case 16: r = launch_view_backward<16>(pts, cam, kp, lt, tiles, bt, io->grad_background, ge, s->env_h, s->env_w, env_inter, st, vl, views[b].camera_model); break;
-            default:
-                snprintf(last_error_buffer(), 512, "%d descriptor channels: the kernels are built for 3, 4, 8 and 16", C);
-                return ADOP_ERR_UNSUPPORTED;
-        }
-        if (r != ADOP_OK) return r;
     }
     if (io->grad_texture && io->grad_texture_interleaved)
     {
@@ -1312,8 +1387,8 @@ extern "C" adop_status adop_raster_backward(const adop_scene* s, const adop_view
     }
     if (env_inter)
     {
-        // [eh,ew,C] -> [C,eh,ew]; the tensor was zeroed above unless the caller accumulates
-        adop_status ds = adop_texture_deinterleave(io->grad_env_map_interleaved, io->grad_env_map, C, s->env_h * s->env_w, 1, stream);
+        // [eh,ew,C] -> [C,eh,ew]
+        adop_status ds = adop_texture_deinterleave(io->grad_env_map_interleaved, io->grad_env_map, C, s->env_h * s->env_w, io->accumulate ? 1 : 0, stream);
         if (ds != ADOP_OK) return ds;
     }
     if (io->normalize)

@@ -418,6 +418,40 @@ def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib
     assert small_list == full_list
 
 
+def test_batch_of_both_camera_models_equals_its_views_one_by_one(cuda_lib):
+    """The views of a batch share launches, in runs of one camera model: each still adds to its own rows of the pose and
+    intrinsics gradients, and a view whose list is not usable does not disturb its neighbours."""
+    cfg = synth.make_config("c2", n_points=70_000, n_views=7, size=(121, 83))
+    a, params, L = cfg["arrays"], cfg["params"], 4
+    coef, theta_max = synth.ocam_world2cam_poly((-20.0, 0.0, 8e-3, -2e-5), rho_max=75.0, degree=7)
+    ocam = np.concatenate([[1, 0, 0, 60, 41], coef]).astype(np.float32)
+    second = a["intrinsics"][0] * 1.05
+    a["intrinsics"] = np.ascontiguousarray(np.stack([a["intrinsics"][0], ocam, second]).astype(np.float32))
+    params.composite_environment_map = 0
+    params.dist_cutoff = float(np.tan(theta_max) * 0.98)
+    rows = [(3, 0), (0, 2), (5, 1), (1, 1), (6, 0), (2, 1), (3, 2)]
+    views = [dict(w=121, h=83, image_index=i, camera_index=c, camera_model=1 if c == 1 else 0) for i, c in rows]
+    scene = to_scene(a)
+    grads = [torch.randn((7, 4, h, w), device="cuda:0") for w, h in capi.layer_sizes(121, 83, L)]
+    keys = ("texture", "background", "points", "pose", "intrinsics", "count_pose", "count_intrinsics")
+    r = PointRasterizer("cuda:0")
+    fwd = r.forward(scene, views, params, L)
+    fwd.visible[4, 2048 + 2] = 1
+    batch = r.backward(scene, params, fwd, grads, normalize=False)
+    total = None
+    for b, view in enumerate(views):
+        one = PointRasterizer("cuda:0")
+        f = one.forward(scene, [view], params, L)
+        for l in range(L):
+            assert torch.equal(f.depths[l][0], fwd.depths[l][b]) and torch.equal(f.weights[l][0], fwd.weights[l][b])
+        g = one.backward(scene, params, f, [x[b:b + 1].contiguous() for x in grads], normalize=False)
+        total = {k: g[k].double() + (total[k] if total else 0.0) for k in keys}
+    for k in keys:
+        # the single views share the batch's drop-out stream only without drop-out, which this configuration does not use
+        close(batch[k], total[k].cpu().numpy(), name=f"batch {k}")
+    assert int((batch["count_pose"] > 0).sum()) == 6 and bool((batch["count_intrinsics"] > 0).all())
+
+
 def test_backward_mode_4(oracle, cuda_lib):
     cfg = synth.make_config("c1", n_points=40_000, size=(96, 96))
     cfg["params"].test_backward_mode = 4
