@@ -544,11 +544,14 @@ __device__ __forceinline__ void async_copy_4(void* smem, const void* gmem)
 }
 __device__ __forceinline__ void async_copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Copies layer LAYER's region of the 2C + 1 planes into shared memory (asynchronously; the caller waits).
+// Copies layer LAYER's region of the 2C + 1 planes into shared memory (asynchronously; the caller waits). A thread takes a place
+// of the region and walks the planes: the place's row, column and bounds are worked out once for all 2C + 1 copies (spread
+// over the threads plane by plane, every copy cost a handful of divisions and pointer selections, a fifth of the
+// kernel's instructions). The layers start at different threads, so that the small regions do not all fall to the first warps.
 template <int C, int LAYER, int STRIDE>
 __device__ __forceinline__ void stage_region(const LayerTable& lt, int view, float* s_tile, int x0, int y0)
 {
-    constexpr int pitch = region_pitch(LAYER), rows = region_rows(LAYER);
+    constexpr int pitch = region_pitch(LAYER), rows = region_rows(LAYER), threads = kTileThreads;
     const int w = lt.w[LAYER], h = lt.h[LAYER];
     const size_t plane = (size_t)w * h;
     const float* weight = view_weight(lt, LAYER, view);
@@ -559,32 +562,40 @@ __device__ __forceinline__ void stage_region(const LayerTable& lt, int view, flo
     const bool vec = (w & 3) == 0 && ((reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(color) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
     if (vec)
     {
-        constexpr int p4 = pitch / 4, per_plane = rows * p4;
-        for (int q = threadIdx.x; q < per_plane * (2 * C + 1); q += kTileThreads)
+        constexpr int p4 = pitch / 4, places = rows * p4, first = (region_offset(LAYER) / 4) % threads;
+        for (int q = ((int)threadIdx.x + threads - first) % threads; q < places; q += threads)
         {
-            const int p = q / per_plane, r = q - p * per_plane;
-            const int row = r / p4, c4 = r - row * p4;
+            const int row = q / p4, c4 = q - row * p4;
             const int gy = sy + row, gx = sx + 4 * c4;
-            if ((unsigned)gy < (unsigned)h && (unsigned)gx < (unsigned)w)
-            {
-                const float* src = p == 0 ? weight : (p <= C ? color + (size_t)(p - 1) * plane : grad + (size_t)(p - 1 - C) * plane);
-                async_copy_16(dst + p * STRIDE + row * pitch + 4 * c4, src + (size_t)gy * w + gx);
-            }
+            if ((unsigned)gy >= (unsigned)h || (unsigned)gx >= (unsigned)w) continue;
+            const size_t at = (size_t)gy * w + gx;
+            float* d = dst + row * pitch + 4 * c4;
+            async_copy_16(d, weight + at);
+            const float* src = color + at;
+#pragma unroll
+            for (int c = 0; c < C; ++c, src += plane) async_copy_16(d + (1 + c) * STRIDE, src);
+            src = grad + at;
+#pragma unroll
+            for (int c = 0; c < C; ++c, src += plane) async_copy_16(d + (1 + C + c) * STRIDE, src);
         }
     }
     else
     {
-        constexpr int per_plane = rows * pitch;
-        for (int q = threadIdx.x; q < per_plane * (2 * C + 1); q += kTileThreads)
+        constexpr int places = rows * pitch, first = region_offset(LAYER) % threads;
+        for (int q = ((int)threadIdx.x + threads - first) % threads; q < places; q += threads)
         {
-            const int p = q / per_plane, r = q - p * per_plane;
-            const int row = r / pitch, col = r - row * pitch;
+            const int row = q / pitch, col = q - row * pitch;
             const int gy = sy + row, gx = sx + col;
-            if ((unsigned)gy < (unsigned)h && (unsigned)gx < (unsigned)w)
-            {
-                const float* src = p == 0 ? weight : (p <= C ? color + (size_t)(p - 1) * plane : grad + (size_t)(p - 1 - C) * plane);
-                async_copy_4(dst + p * STRIDE + row * pitch + col, src + (size_t)gy * w + gx);
-            }
+            if ((unsigned)gy >= (unsigned)h || (unsigned)gx >= (unsigned)w) continue;
+            const size_t at = (size_t)gy * w + gx;
+            float* d = dst + q;
+            async_copy_4(d, weight + at);
+            const float* src = color + at;
+#pragma unroll
+            for (int c = 0; c < C; ++c, src += plane) async_copy_4(d + (1 + c) * STRIDE, src);
+            src = grad + at;
+#pragma unroll
+            for (int c = 0; c < C; ++c, src += plane) async_copy_4(d + (1 + C + c) * STRIDE, src);
         }
     }
 }
