@@ -24,7 +24,7 @@
 namespace adop {
 
 // ------------------------------------------------------------------------------------------------------
-// K4: preparation pass over the pyramid pixels of one view (all-points path only; returns at once behind a usable list).
+// K4: preparation pass over the pyramid pixels of one view (all-points path only).
 //  * writes the interleaved record [I_0..I_C-1 | G_0..G_C-1] (I = the forward image before the environment-map
 //    composite: the background colour where nothing was blended, PointRenderer.cu:1523);
 //  * sums the gradient of the background colour over uncovered pixels (CombineAndFillBackward, :851-900);
@@ -1155,7 +1155,7 @@ __global__ void k_normalize_intrinsics(float* g, const float* cnt, int n, int co
 }
 
 // ------------------------------------------------------------------------------------------------------
-constexpr int kTileWaves = 2, kChainWaves = 1;
+constexpr int kTileWaves = 2;
 static int blocks_per_view(int resident, int waves, int views, int most)
 {
     int n = (resident * waves + views - 1) / views;
@@ -1196,7 +1196,10 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
     {
         // the chain blocks get five eighths of the blocks when both parts have work (measured: between a half and three quarters
         // the kernel's time is flat, beyond it rises quickly)
-        const int per_view = blocks_per_view(g, kChainWaves, views, 1 << 30);
+        // A batch of two to four views gets twice the resident blocks: its views differ in work, and a block row that is done early
+    // leaves room for the next (chain and holes, one wave and two: four 4K views 1655 and 1495 us, sixteen 1080p views 856 and
+    // 869, eight 568 and 646, one 512 x 512 view 16.9 and 18.9).
+    const int per_view = blocks_per_view(g, views >= 2 && views <= 4 ? 2 : 1, views, 1 << 30);
         int chain_blocks = want_geo ? (hole_need ? per_view * 5 / 8 : per_view) : 0;
         if (want_geo && chain_blocks < 1) chain_blocks = 1;
         if (chain_blocks > tt.n_tiles) chain_blocks = tt.n_tiles;
