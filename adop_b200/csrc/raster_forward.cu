@@ -146,7 +146,7 @@ struct CandOut
     int keep_dropped;     // the visible list wants dropped points too (ghost-gradient mode)
 };
 template <int L, bool PLAIN, int V, bool CAND>
-__global__ void __launch_bounds__(kBlock, PLAIN ? 8 : 4) k_depth_prepass(PointStreams pts, ChunkSchedule sched, const ViewCam* __restrict__ camp, KernelParams kp,
+__global__ void __launch_bounds__(kBlock, PLAIN || !CAND ? 8 : 4) k_depth_prepass(PointStreams pts, ChunkSchedule sched, const ViewCam* __restrict__ camp, KernelParams kp,
                                                            LayerTable lt, CandOut co)
 {
     const bool use_normal = PLAIN ? false : kp.check_normal != 0;
@@ -658,7 +658,7 @@ struct ForwardPlan
     int32_t* list_base;   // null = no visible list
     int w, h;             // layer-0 size (geometry of the visible list)
     char* large;          // large region of a full workspace (candidate streams), null = small workspace
-    bool stream_plain;    // candidate streams also for pinhole views without normal test and radius rule
+    bool omnidirectional, dense;  // a view of the omnidirectional model; many points per pixel
     LargeRegion lr;
     size_t cand_view_stride;  // records per candidate stream
     TileTable tiles;
@@ -683,7 +683,8 @@ static adop_status launch_group_forward_impl(const PointStreams& pts, const adop
     const int need = (pts.n + kBlock - 1) / kBlock;
     // Candidate streams pay where the projection is expensive (omnidirectional model, normal test, radius rule) or most points
     // of a pixel are hidden; the radius rule's layer count shares the id word of a record.
-    const bool cand = plan.large != nullptr && (plan.stream_plain || !PLAIN) && (!kp.drop_out_points_by_radius || pts.n <= kCandIdMask);
+    const bool cand = plan.large != nullptr && (plan.omnidirectional || !PLAIN || (plan.dense && views > 1)) &&
+                      (!kp.drop_out_points_by_radius || pts.n <= kCandIdMask);
     const bool emit = plan.list_base != nullptr;
     const int g_position = emit ? g_blend_emit : g_blend;
     int grid_blend = g_position < need ? g_position : (need < 1 ? 1 : need);
@@ -1011,9 +1012,12 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     // Pinhole views, no normal test, no radius rule: the streams cost the prepass the depth reads of the finest layer and the
     // records, and save the blend kernel the hidden points. Per view at 1080p, four layers, four channels, prepass + blend: 4.8
     // points per pixel 196 us without and 205 us with streams, 14.5 points per pixel 455 and 361 us; 4K, six layers, eight
-    // channels, 6.0 points per pixel 1515 and 1391 us.
-    plan.stream_plain = (double)N >= 5.5 * (double)w0 * (double)h0;
-    for (int b = 0; b < B; ++b) plan.stream_plain = plan.stream_plain || views[b].camera_model == ADOP_CAMERA_OCAM;
+    // channels, 6.0 points per pixel 1515 and 1391 us. A view on its own gains nothing (3.4 M points, 509 x 335) or loses (frame
+    // of 2.7 M points, 313 x 307: 142 and 173 us): the position is not shared with other views, and all its threads read
+    // the cleared planes of a small image before anyone's minimum has arrived.
+    plan.dense = (double)N >= 5.5 * (double)w0 * (double)h0;
+    plan.omnidirectional = false;
+    for (int b = 0; b < B; ++b) plan.omnidirectional = plan.omnidirectional || views[b].camera_model == ADOP_CAMERA_OCAM;
     plan.lr = lr;
     plan.cand_view_stride = entry_capacity(N);
     // the pose and intrinsics tensors live on the device; the per-view cameras are gathered there, a chunk at a time
