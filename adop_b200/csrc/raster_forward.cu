@@ -658,7 +658,7 @@ struct ForwardPlan
     int32_t* list_base;   // null = no visible list
     int w, h;             // layer-0 size (geometry of the visible list)
     char* large;          // large region of a full workspace (candidate streams), null = small workspace
-    bool omnidirectional, dense;  // a view of the omnidirectional model; many points per pixel
+    bool omnidirectional, dense, not_tiny;  // a view of the omnidirectional model; many points per pixel; 2^15 pixels or more
     LargeRegion lr;
     size_t cand_view_stride;  // records per candidate stream
     TileTable tiles;
@@ -683,7 +683,7 @@ static adop_status launch_group_forward_impl(const PointStreams& pts, const adop
     const int need = (pts.n + kBlock - 1) / kBlock;
     // Candidate streams pay where the projection is expensive (omnidirectional model, normal test, radius rule) or most points
     // of a pixel are hidden; the radius rule's layer count shares the id word of a record.
-    const bool cand = plan.large != nullptr && (plan.omnidirectional || !PLAIN || (plan.dense && views > 1)) &&
+    const bool cand = plan.large != nullptr && (plan.omnidirectional || (!PLAIN && plan.not_tiny) || (plan.dense && views > 1)) &&
                       (!kp.drop_out_points_by_radius || pts.n <= kCandIdMask);
     const bool emit = plan.list_base != nullptr;
     const int g_position = emit ? g_blend_emit : g_blend;
@@ -1016,6 +1016,10 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     // of 2.7 M points, 313 x 307: 142 and 173 us): the position is not shared with other views, and all its threads read
     // the cleared planes of a small image before anyone's minimum has arrived.
     plan.dense = (double)N >= 5.5 * (double)w0 * (double)h0;
+    // With the normal test or the radius rule the projection is dear and the streams pay, but not on tiny images, where the
+    // atomics on a few pixels are what takes the time (training steps of two views: 178 x 144, 750 k points 279 us without and
+    // 326 us with streams; 201 x 184, 1.1 M points 251 and 218 us).
+    plan.not_tiny = (long long)w0 * h0 >= (1 << 15);
     plan.omnidirectional = false;
     for (int b = 0; b < B; ++b) plan.omnidirectional = plan.omnidirectional || views[b].camera_model == ADOP_CAMERA_OCAM;
     plan.lr = lr;

@@ -209,7 +209,7 @@ size_t adop_raster_workspace_bytes(int32_t w, int32_t h, int32_t layers, int32_t
  * accumulators for such a group (24 MB at most). With a workspace of at least this size
  *   - the depth prepass can hand the projected points that may still be accepted to the blend kernel, which then neither
  *     reads the cloud again nor projects a second time; the library does so where it pays: omnidirectional views, normal
- *     test or radius rule in use, or several views and 5.5 points of the cloud per pixel and more;
+ *     test or radius rule in use and an image of 2^15 pixels or more, or several views and 5.5 points of the cloud per pixel and more;
  *   - the views of a group of small ones are blended and resolved in one launch each.
  * Same results either way. The host layers of this library ask for it and fall back to the small workspace where the
  * device has no room. */

@@ -379,9 +379,10 @@ def test_small_workspace_matches_full_workspace(cuda_lib):
     (1, (40, 24), 1, 1, False, 0, False),            # one point, one layer
     (257, (33, 17), 3, 3, False, 0, False),          # one point past a chunk, odd planes
     (90_011, (101, 57), 5, 4, False, 0, False),      # 15 points per pixel, two groups of views
-    (90_011, (101, 57), 5, 4, True, 0, False),       # normal test and radius rule: the record carries the layer count
-    (90_011, (101, 57), 4, 5, True, 1, False),       # dropped points stay in the stream for the visible list
-    (60_000, (64, 48), 2, 5, True, 0, True),         # drop-out decisions from the caller's mask
+    (200_011, (257, 131), 5, 4, True, 0, False),     # normal test and radius rule: the record carries the layer count
+    (200_011, (257, 131), 4, 5, True, 1, False),     # dropped points stay in the stream for the visible list
+    (60_000, (64, 48), 2, 5, True, 0, False),        # a tiny image: positions on both sides
+    (150_000, (256, 128), 2, 5, True, 0, True),      # drop-out decisions from the caller's mask
 ])
 def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib, points, size, views, layers, rule, ghost, mask):
     """Full workspace (the prepass drops points that already fail the depth test everywhere) against the small one (every
