@@ -311,7 +311,7 @@ static_assert(kMaxLayers <= 8, "three bits hold the layer count");
 constexpr size_t kGroupAccumBytes = (size_t)24 << 20;
 struct LargeRegion
 {
-    size_t cand_rec, cand_count, accum, total;  // byte offsets from the region's start (forward)
+    size_t accum, accum_end, cand_rec, cand_count, total;  // byte offsets from the region's start (forward)
     int accum_views;
 };
 inline LargeRegion large_region_layout(int num_points, int num_views, size_t accum_bytes)
@@ -319,12 +319,13 @@ inline LargeRegion large_region_layout(int num_points, int num_views, size_t acc
     const int v = num_views < kCandViews ? (num_views < 1 ? 1 : num_views) : kCandViews;
     const size_t cap = entry_capacity(num_points);
     LargeRegion r;
-    r.cand_rec = 0;
-    r.cand_count = r.cand_rec + (size_t)v * cap * 16;
-    r.accum = r.cand_count + (((size_t)v * kVisibleSegments * sizeof(int) + 255) & ~(size_t)255);
     r.accum_views = 1;
     while (r.accum_views < v && (size_t)(r.accum_views + 1) * accum_bytes <= kGroupAccumBytes) ++r.accum_views;
-    r.total = r.accum + (r.accum_views > 1 ? (size_t)r.accum_views * accum_bytes : 0) + 256;
+    r.accum = 0;
+    r.accum_end = r.accum_views > 1 ? ((size_t)r.accum_views * accum_bytes + 255) & ~(size_t)255 : 0;
+    r.cand_rec = r.accum_end;
+    r.cand_count = r.cand_rec + (size_t)v * cap * 16;
+    r.total = r.cand_count + (((size_t)v * kVisibleSegments * sizeof(int) + 255) & ~(size_t)255) + 256;
     return r;
 }
 

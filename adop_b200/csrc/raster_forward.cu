@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(kBlock) k_texture_deinterleave(const float* __
 // and does not project again: it sees the same float x, y, depth, hence takes the same decisions bit for bit.
 // A point is left out when it already fails the fuzzy depth test on every layer it lands in, against the depth planes as
 // they are at that moment: depths only decrease, so the final planes refuse it too. (Also left out: dropped points, when
-// nothing downstream wants them.) The test needs the depth of every layer, so all reads go out together, the finest
-// layer's too; what that costs here is less than what the shorter stream saves behind it.
+// nothing downstream wants them.) The test needs the depth of every layer, the finest one's too; all reads go out
+// together, unless the coarsest layer is tiny (CandOut::layer_by_layer).
 struct CandOut
 {
     float4* rec;          // view v: rec + v * view_stride
@@ -144,6 +144,7 @@ struct CandOut
     size_t view_stride;   // records per view
     int seg_cap;          // records per block segment
     int keep_dropped;     // the visible list wants dropped points too (ghost-gradient mode)
+    int layer_by_layer;   // read a layer's depth just before its minimum (without normal test and radius rule)
 };
 template <int L, bool PLAIN, int V, bool CAND>
 __global__ void __launch_bounds__(kBlock, PLAIN || !CAND ? 8 : 4) k_depth_prepass(PointStreams pts, ChunkSchedule sched, const ViewCam* __restrict__ camp, KernelParams kp,
@@ -184,7 +185,20 @@ __global__ void __launch_bounds__(kBlock, PLAIN || !CAND ? 8 : 4) k_depth_prepas
             {
                 float x = q.x, y = q.y, rad = q.radius_px;
                 const int zi = __float_as_int(q.z);
-                if (CAND)
+                if (CAND && PLAIN && co.layer_by_layer)
+                {
+#pragma unroll
+                    for (int l = 0; l < L; ++l, x *= 0.5f, y *= 0.5f)
+                    {
+                        const int px = round_half_even_bounded(x), py = round_half_even_bounded(y);
+                        if ((unsigned)px >= (unsigned)lt.w[l] || (unsigned)py >= (unsigned)lt.h[l]) continue;
+                        float* dst = lt.depth[l] + ((unsigned)(v * lt.h[l] + py) * (unsigned)lt.w[l] + (unsigned)px);
+                        const float d = __ldcg(dst);
+                        if (q.z < d) atomicMin(reinterpret_cast<int*>(dst), zi);
+                        if (!(q.z > d * kp.depth_accept_plus_one)) keep = true;
+                    }
+                }
+                else if (CAND)
                 {
                     unsigned lin[L];
                     float d[L];
@@ -655,10 +669,12 @@ struct ForwardPlan
     size_t accum_stride;  // floats from accumulator to accumulator
     int blend_views;      // views that are blended in one launch
     bool env;
+    const adop_render_params* rp;
     int32_t* list_base;   // null = no visible list
     int w, h;             // layer-0 size (geometry of the visible list)
-    char* large;          // large region of a full workspace (candidate streams), null = small workspace
-    bool omnidirectional, dense, not_tiny;  // a view of the omnidirectional model; many points per pixel; 2^15 pixels or more
+    char* large;          // large region of a full workspace (candidate streams); null: no room for them
+    bool omnidirectional;    // a view of the omnidirectional model
+    bool coarse_layer_tiny;  // see CandOut::layer_by_layer
     LargeRegion lr;
     size_t cand_view_stride;  // records per candidate stream
     TileTable tiles;
@@ -667,11 +683,49 @@ struct ForwardPlan
     unsigned char* touched_texels;
 };
 
+// Neither the normal test (or no normals) nor the radius rule: the common case, kernels without that code.
+static bool plain_projection(const adop_scene* s, const adop_render_params* rp)
+{
+    const bool normals = s->normal || (s->outlier_position && s->num_outliers > 0 && s->outlier_normal);
+    return !(rp->check_normal && normals) && !rp->drop_out_points_by_radius;
+}
+
+// Does a group of `views` views go through candidate streams (given the room)? They cost the prepass the depth reads of the
+// finest layer and the records, and save the blend kernel the hidden points and every projection. Both routes of one build
+// against each other, prepass + blend, positions : streams, four layers and channels where not said otherwise:
+//  * omnidirectional model: the projection is dear, streams always. 30 M points, one 1080p view 689 : 474 us; 1 M, 320 x 240, two
+//    views 74 : 64 us; at its worst (2.3 M points, 1237 x 731, four views) 303 : 303 us.
+//  * pinhole, no normal test, no radius rule: the points that hide behind others have to pay for the records and for filling the
+//    planes. Four views at 1080p, 4.5 points per pixel 752 : 788 us, 5.5 856 : 864, 6 925 : 897, 9 1265 : 1099; 960 x 540, 5 points per pixel
+//    229 : 233 us, 7 284 : 269; 640 x 480, 6.5 179 : 185, 9.8 239 : 226; 320 x 240, 3.9 64 : 66, 13 109 : 97. With 4K, six layers and
+//    eight channels at 6 points per pixel four views gain (5.80 : 5.57 ms) and two lose (2.68 : 2.78 ms). A view on its own does not
+//    share its positions with others and stays with them: it gains on large dense images (960 x 540, 14 points per pixel 152 : 130 us)
+//    and loses on small ones (frame of 313 x 307, five layers, 28 points per pixel 130 : 181 us).
+//  * normal test or radius rule: the projection is dear again, but the prepass with streams runs with half the warps. Groups: 512 x 512, four
+//    views, 3.1 points per pixel 81 : 89 us, 8.4 161 : 163, 13 232 : 218; 320 x 240, 1 M points 87 : 87; 178 x 144, 0.6 M 58 : 56,
+//    2.2 M 144 : 112; 1080p, 1.7 points per pixel 356 : 387, 4.8 (five layers) 805 : 728. One view: 512 x 512, 0.8 M points 38 : 36; 1080p,
+//    1.5 M points, radius rule 79 : 87.
+// The radius rule's layer count shares the id word of a record, which limits the cloud.
+static bool streams_pay(const adop_scene* s, const adop_render_params* rp, bool omnidirectional, int w, int h, int views)
+{
+    const long long n = s->num_points, pixels = (long long)w * h;
+    if (rp->drop_out_points_by_radius && n > kCandIdMask) return false;
+    if (omnidirectional) return true;
+    if (plain_projection(s, rp)) return views > 1 && 2 * n >= 11 * pixels + 500000;
+    return views > 1 ? n >= 4 * pixels + 700000 : n >= 2 * pixels;
+}
+static bool any_omnidirectional(const adop_view* views, int B)
+{
+    for (int b = 0; b < B; ++b)
+        if (views[b].camera_model == ADOP_CAMERA_OCAM) return true;
+    return false;
+}
+
 // One group of up to kCandViews consecutive views, `view` the first: depth prepass of all of them, then blend and resolve,
-// plan.blend_views at a time. lt, kp and cams are the first view's.
+// plan.blend_views at a time. lt, kp and cams are the first view's; cand: with candidate streams.
 template <int L, int C, bool PLAIN>
 static adop_status launch_group_forward_impl(const PointStreams& pts, const adop_scene* s, const ViewCam* cams, const KernelParams& kp,
-                                             const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int views)
+                                             const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int views, bool cand)
 {
     static const int g_depth = resident_grid(k_depth_prepass<L, PLAIN, 4, false>, 1ll << 40);
     static const int g_depth_cand = resident_grid(k_depth_prepass<L, PLAIN, 4, true>, 1ll << 40);
@@ -681,10 +735,6 @@ static adop_status launch_group_forward_impl(const PointStreams& pts, const adop
     static const int g_blend_cand_emit = resident_grid(k_blend<L, C, true, true, true>, 1ll << 40);
     static const int g_resolve = resident_grid(k_resolve<C>, 1ll << 40);
     const int need = (pts.n + kBlock - 1) / kBlock;
-    // Candidate streams pay where the projection is expensive (omnidirectional model, normal test, radius rule) or most points
-    // of a pixel are hidden; the radius rule's layer count shares the id word of a record.
-    const bool cand = plan.large != nullptr && (plan.omnidirectional || (!PLAIN && plan.not_tiny) || (plan.dense && views > 1)) &&
-                      (!kp.drop_out_points_by_radius || pts.n <= kCandIdMask);
     const bool emit = plan.list_base != nullptr;
     const int g_position = emit ? g_blend_emit : g_blend;
     int grid_blend = g_position < need ? g_position : (need < 1 ? 1 : need);
@@ -709,6 +759,7 @@ static adop_status launch_group_forward_impl(const PointStreams& pts, const adop
     co.view_stride = plan.cand_view_stride;
     co.seg_cap = seg_cap;
     co.keep_dropped = emit && kp.ghost_gradients;
+    co.layer_by_layer = plan.coarse_layer_tiny;
 #define ADOP_PREPASS(VV)                                                                                                         \
     if (cand) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, true><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cams, kp, lt, co))); \
     else ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<grid_depth, kBlock, 0, st>>>(pts, make_chunk_schedule(pts.n, grid_depth), cams, kp, lt, co)));
@@ -727,7 +778,7 @@ static adop_status launch_group_forward_impl(const PointStreams& pts, const adop
     {
         const int og = oneed < g_depth ? oneed : g_depth;
         CandOut none;
-        none.rec = nullptr; none.count = nullptr; none.view_stride = 0; none.seg_cap = 0; none.keep_dropped = 0;
+        none.rec = nullptr; none.count = nullptr; none.view_stride = 0; none.seg_cap = 0; none.keep_dropped = 0; none.layer_by_layer = 0;
 #define ADOP_PREPASS_OUT(VV) ADOP_LAUNCH("k_depth_prepass", st, (k_depth_prepass<L, PLAIN, VV, false><<<og, kBlock, 0, st>>>(op, make_chunk_schedule(op.n, og), cams, kp, lt, none)))
         switch (views)
         {
@@ -798,10 +849,9 @@ template <int L, int C>
 static adop_status launch_group_forward(const PointStreams& pts, const adop_scene* s, const ViewCam* cams, const KernelParams& kp,
                                         const LayerTable& lt, const ForwardPlan& plan, cudaStream_t st, int view, int views)
 {
-    // the common case - no normal test (or no normals) and no radius drop-out - gets kernels without that code
-    const bool plain = !(kp.check_normal && (pts.normal || plan.outliers.normal)) && !kp.drop_out_points_by_radius;
-    return plain ? launch_group_forward_impl<L, C, true>(pts, s, cams, kp, lt, plan, st, view, views)
-                 : launch_group_forward_impl<L, C, false>(pts, s, cams, kp, lt, plan, st, view, views);
+    const bool cand = plan.large != nullptr && streams_pay(s, plan.rp, plan.omnidirectional, plan.w, plan.h, views);
+    return plain_projection(s, plan.rp) ? launch_group_forward_impl<L, C, true>(pts, s, cams, kp, lt, plan, st, view, views, cand)
+                                        : launch_group_forward_impl<L, C, false>(pts, s, cams, kp, lt, plan, st, view, views, cand);
 }
 
 template <int C>
@@ -844,16 +894,34 @@ static size_t workspace_large_offset(int32_t w, int32_t h, int32_t layers, int32
     return (adop_raster_workspace_bytes(w, h, layers, channels) + 255) & ~(size_t)255;
 }
 
+// floats of one view's accumulator (AccumLayout: with a multiple of four channels the counts go into the weight images)
+static size_t accumulator_floats(int w, int h, int layers, int channels)
+{
+    LayerTable lt;
+    fill_layer_dims(w, h, layers, &lt);
+    return (size_t)lt.rec_off[kMaxLayers] * (channels % 4 == 0 ? channels : record_floats(channels));
+}
+
 extern "C" size_t adop_raster_workspace_bytes_full(int32_t num_points, int32_t num_views, int32_t w, int32_t h, int32_t layers,
                                                    int32_t channels)
 {
     const size_t small = adop_raster_workspace_bytes(w, h, layers, channels);
     if (small == 0 || num_points < 0 || num_views <= 0) return 0;
-    // candidate streams of a group of views, accumulators of a group of small ones
-    LayerTable lt;
-    fill_layer_dims(w, h, layers, &lt);
-    const size_t accum_bytes = (size_t)lt.rec_off[kMaxLayers] * (channels % 4 == 0 ? channels : record_floats(channels)) * sizeof(float);
-    return workspace_large_offset(w, h, layers, channels) + large_region_layout(num_points, num_views, accum_bytes).total;
+    return workspace_large_offset(w, h, layers, channels) +
+           large_region_layout(num_points, num_views, accumulator_floats(w, h, layers, channels) * sizeof(float)).total;
+}
+
+extern "C" size_t adop_raster_forward_workspace_bytes(const adop_scene* s, const adop_view* views, int32_t num_views, const adop_render_params* rp,
+                                                      int32_t layers)
+{
+    if (validate_common(s, views, num_views, rp, layers) != ADOP_OK) return 0;
+    const int w = views[0].w, h = views[0].h;
+    const bool omnidirectional = any_omnidirectional(views, num_views);
+    for (int b = 0; b < num_views; b += kCandViews)
+        if (streams_pay(s, rp, omnidirectional, w, h, num_views - b < kCandViews ? num_views - b : kCandViews))
+            return adop_raster_workspace_bytes_full(s->num_points, num_views, w, h, layers, s->channels);
+    const LargeRegion lr = large_region_layout(s->num_points, num_views, accumulator_floats(w, h, layers, s->channels) * sizeof(float));
+    return lr.accum_views > 1 ? workspace_large_offset(w, h, layers, s->channels) + lr.accum_end : adop_raster_workspace_bytes(w, h, layers, s->channels);
 }
 
 extern "C" adop_status adop_texture_interleave(const float* texture, float* out, int32_t channels, int32_t num_texels, void* stream)
@@ -925,22 +993,20 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     fill_layer_dims(w0, h0, L, &base);
     ViewCam* cams = static_cast<ViewCam*>(io->workspace);
     const bool split = C % 4 == 0;  // AccumLayout: colour sums only, the counts go into the weight images
-    const size_t accum_floats = (size_t)base.rec_off[kMaxLayers] * (split ? C : record_floats(C));
-    // A workspace of adop_raster_workspace_bytes_full has a large region behind the pixel records: candidate streams from
-    // the depth prepass to the blend kernel, and accumulators for a group of views where they are small.
+    const size_t accum_floats = accumulator_floats(w0, h0, L, C);
+    // A larger workspace has a region behind the pixel records: accumulators for a group of views where they are small, and
+    // behind them the candidate streams from the depth prepass to the blend kernel. The call takes what it is given.
     float* accum = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + kCamRegionBytes);
     int accum_views = 1;
     char* large = nullptr;
     const LargeRegion lr = large_region_layout(N, B, accum_floats * sizeof(float));
-    if (io->workspace_bytes >= adop_raster_workspace_bytes_full(N, B, w0, h0, L, C))
+    const size_t large_offset = workspace_large_offset(w0, h0, L, C);
+    if (lr.accum_views > 1 && io->workspace_bytes >= large_offset + lr.accum_end)
     {
-        large = static_cast<char*>(io->workspace) + workspace_large_offset(w0, h0, L, C);
-        if (lr.accum_views > 1)
-        {
-            accum = reinterpret_cast<float*>(large + lr.accum);
-            accum_views = lr.accum_views;
-        }
+        accum = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + large_offset + lr.accum);
+        accum_views = lr.accum_views;
     }
+    if (io->workspace_bytes >= adop_raster_workspace_bytes_full(N, B, w0, h0, L, C)) large = static_cast<char*>(io->workspace) + large_offset;
     const int sms = sm_count();
     // the accumulator, depth.fill_(100000) (PointRenderer.cu:1045), the counts, the cursors of the visible lists (colours, and
     // the weights of the other layout, are written by the resolve kernel)
@@ -987,6 +1053,7 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     plan.accum_stride = accum_floats;
     plan.blend_views = accum_views;
     plan.env = env;
+    plan.rp = rp;
     plan.list_base = io->visible_list;
     plan.w = w0; plan.h = h0;
     plan.tiles = make_tile_table(w0, h0, N);
@@ -1009,19 +1076,13 @@ extern "C" adop_status adop_raster_forward(const adop_scene* s, const adop_view*
     plan.outliers.index = s->outlier_index;
     plan.outliers.n = s->outlier_position ? s->num_outliers : 0;
     plan.large = large;
-    // Pinhole views, no normal test, no radius rule: the streams cost the prepass the depth reads of the finest layer and the
-    // records, and save the blend kernel the hidden points. Per view at 1080p, four layers, four channels, prepass + blend: 4.8
-    // points per pixel 196 us without and 205 us with streams, 14.5 points per pixel 455 and 361 us; 4K, six layers, eight
-    // channels, 6.0 points per pixel 1515 and 1391 us. A view on its own gains nothing (3.4 M points, 509 x 335) or loses (frame
-    // of 2.7 M points, 313 x 307: 142 and 173 us): the position is not shared with other views, and all its threads read
-    // the cleared planes of a small image before anyone's minimum has arrived.
-    plan.dense = (double)N >= 5.5 * (double)w0 * (double)h0;
-    // With the normal test or the radius rule the projection is dear and the streams pay, but not on tiny images, where the
-    // atomics on a few pixels are what takes the time (training steps of two views: 178 x 144, 750 k points 279 us without and
-    // 326 us with streams; 201 x 184, 1.1 M points 251 and 218 us).
-    plan.not_tiny = (long long)w0 * h0 >= (1 << 15);
-    plan.omnidirectional = false;
-    for (int b = 0; b < B; ++b) plan.omnidirectional = plan.omnidirectional || views[b].camera_model == ADOP_CAMERA_OCAM;
+    // With streams the prepass reads the depth of all layers before the first minimum goes out. While a small image is filled,
+    // every resident thread then finds the cleared planes and they all queue up at the few pixels of the coarsest layer; reading a layer just
+    // before its own minimum spreads them out. Prepass + blend together : layer by layer, 1 M points: two views of 178 x 144, five layers
+    // (99 pixels) 222 : 115 us; four of 320 x 240, four layers (1200 pixels) 107 : 97; from 2000 pixels on the waits cost more (four 1080p
+    // views, six layers, 1980 pixels, 20 M points 1350 : 1364 us, four layers 1163 : 1190).
+    plan.coarse_layer_tiny = (long long)base.w[L - 1] * base.h[L - 1] < 1500;
+    plan.omnidirectional = any_omnidirectional(views, B);
     plan.lr = lr;
     plan.cand_view_stride = entry_capacity(N);
     // the pose and intrinsics tensors live on the device; the per-view cameras are gathered there, a chunk at a time

@@ -205,16 +205,21 @@ void adop_render_params_default(adop_render_params* p);
 /* Bytes of scratch that forward/backward need for views of w x h with `layers` layers and `channels`
  * descriptor channels. Replaces the size-keyed PointRendererCache (PointRenderer.h:96-157). */
 size_t adop_raster_workspace_bytes(int32_t w, int32_t h, int32_t layers, int32_t channels);
-/* The same plus 16 bytes per point and view of a group of up to four views (about 64 N bytes) and, where they are small,
- * accumulators for such a group (24 MB at most). With a workspace of at least this size
- *   - the depth prepass can hand the projected points that may still be accepted to the blend kernel, which then neither
- *     reads the cloud again nor projects a second time; the library does so where it pays: omnidirectional views, normal
- *     test or radius rule in use and an image of 2^15 pixels or more, or several views and 5.5 points of the cloud per pixel and more;
- *   - the views of a group of small ones are blended and resolved in one launch each.
- * Same results either way. The host layers of this library ask for it and fall back to the small workspace where the
- * device has no room. */
+/* The same plus, where they are small, accumulators for a group of up to four views (24 MB at most) and 16 bytes per point and
+ * view of such a group (about 64 N bytes): room for everything that any forward pass of this size can use.
+ *   - With the accumulators the views of a group of small ones are blended and resolved in one launch each.
+ *   - With the 16 bytes per point and view the depth prepass can hand the projected points that may still be accepted to the
+ *     blend kernel, which then neither reads the cloud again nor projects a second time. The library does so where it pays:
+ *     omnidirectional views; several views with 5.5 points of the cloud per pixel (and a quarter of a million) or more; with normal test or
+ *     radius rule one view with 2 points per pixel, several with 4 (and 0.7 million) or more.
+ * Same results either way. */
 size_t adop_raster_workspace_bytes_full(int32_t num_points, int32_t num_views, int32_t w, int32_t h, int32_t layers,
                                         int32_t channels);
+/* The bytes of workspace that adop_raster_forward makes use of for exactly these arguments: between the two sizes above,
+ * without the parts that this call would not read. 0 for arguments that adop_raster_forward refuses. Reads nothing on the
+ * device. */
+size_t adop_raster_forward_workspace_bytes(const adop_scene* scene, const adop_view* views, int32_t num_views, const adop_render_params* params,
+                                           int32_t layers);
 
 /* [C,T] -> [T,C] (and back, optionally adding to `out`): the descriptor tensor keeps the reference's planar layout
  * at the boundary (NeuralTexture.h:62); these build the interleaved working copy the kernels prefer. */

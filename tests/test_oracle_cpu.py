@@ -495,6 +495,52 @@ def test_c_abi_library_exports_every_declared_symbol():
     assert lib.adop_raster_workspace_bytes(0, 1080, 4, 4) == 0
 
 
+def _forward_workspace(points, size, views, layers=4, channels=4, model=0, rule=False, normals=False):
+    """(what a forward pass of these arguments makes use of, small size, full size); nothing is read on a device."""
+    lib = capi.load_library()
+    sc, params = capi.AdopScene(), capi.default_render_params()
+    sc.num_points = sc.num_texels = points
+    sc.channels, sc.num_images, sc.num_cameras, sc.intrinsics_cols = channels, 1, 1, 13
+    sc.position = sc.texture = sc.background = sc.poses = sc.intrinsics = 4096  # any address
+    sc.normal = 4096 if normals else None
+    params.drop_out_points_by_radius = int(rule)
+    va = capi.make_views([dict(w=size[0], h=size[1], image_index=0, camera_model=model)] * views)
+    used = lib.adop_raster_forward_workspace_bytes(ctypes.byref(sc), va, views, ctypes.byref(params), layers)
+    return (used, lib.adop_raster_workspace_bytes(*size, layers, channels),
+            lib.adop_raster_workspace_bytes_full(points, views, *size, layers, channels))
+
+
+@pytest.mark.parametrize("points,size,views,kw,streams", [
+    # groups of plain pinhole views: small images need more points per pixel than large ones
+    (300_000, (178, 144), 2, {}, False), (720_000, (178, 144), 2, {}, True), (690_000, (320, 240), 4, {}, True), (600_000, (320, 240), 4, {}, False),
+    (10_000_000, (1920, 1080), 16, {}, False), (12_000_000, (1920, 1080), 16, {}, True), (50_000_000, (3840, 2160), 4, dict(layers=6, channels=8), True),
+    # one view keeps to its positions
+    (100_000_000, (1920, 1080), 1, {}, False),
+    # ... unless its projection is dear
+    (100_000_000, (1920, 1080), 1, dict(model=1), True), (1000, (64, 48), 1, dict(model=1), True),
+    (3_000_000, (512, 512), 4, dict(rule=True, normals=True), True), (1_000_000, (512, 512), 4, dict(rule=True), False),
+    (1_000_000, (512, 512), 1, dict(normals=True), True), (1_000_000, (1920, 1080), 1, dict(rule=True), False),
+    # the radius rule's records hold 28-bit point numbers
+    (1 << 28, (512, 512), 4, dict(rule=True), False), ((1 << 28) - 1, (512, 512), 4, dict(rule=True), True), (1 << 28, (512, 512), 4, dict(normals=True), True),
+])
+def test_forward_workspace_follows_the_rule_for_candidate_streams(points, size, views, kw, streams):
+    used, small, full = _forward_workspace(points, size, views, **kw)
+    assert (used == full) == streams and small <= used <= full
+    if not streams:
+        assert used <= small + 256 + (24 << 20)
+
+
+def test_forward_workspace_without_streams_holds_the_group_accumulators_only():
+    used, small, full = _forward_workspace(500_000, (512, 512), 4)
+    assert used - small >= 4 * (512 * 512 + 256 * 256 + 128 * 128 + 64 * 64) * 16 and used < full
+    for views, size in ((1, (512, 512)), (4, (1920, 1080))):  # nothing to group; accumulators too large to group
+        used, small, full = _forward_workspace(500_000, size, views)
+        assert used == small
+    lib = capi.load_library()
+    assert lib.adop_raster_forward_workspace_bytes(None, None, 1, None, 4) == 0
+    assert _forward_workspace(1000, (4, 4), 1, layers=4)[0] == 0  # the coarsest layer would be empty
+
+
 def test_struct_sizes_match_the_header():
     """ctypes mirrors must have the C layout (compiled probe with the system compiler)."""
     import subprocess

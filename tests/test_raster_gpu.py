@@ -6,12 +6,14 @@ multi-splat pixels, all gradients) per element within |a - b| <= 1e-4 |b| + 1e-5
 ordering differs, and a floor of 1e-5 of the tensor's largest magnitude for elements whose terms cancel. Results that
 involve no atomics are held to 1e-5 relative (RTOL_EXACT_ORDER).
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from adop_b200 import capi, synth
-from adop_b200.raster import PointRasterizer, Scene
+from adop_b200.raster import PointRasterizer, Scene, fill_scene_struct
 
 pytestmark = pytest.mark.gpu
 
@@ -375,22 +377,39 @@ def test_small_workspace_matches_full_workspace(cuda_lib):
         close(ba[k], bb[k].cpu().numpy(), name=f"small vs full grad {k}")
 
 
-@pytest.mark.parametrize("points,size,views,layers,rule,ghost,mask", [
-    (1, (40, 24), 1, 1, False, 0, False),            # one point, one layer
-    (257, (33, 17), 3, 3, False, 0, False),          # one point past a chunk, odd planes
-    (90_011, (101, 57), 5, 4, False, 0, False),      # 15 points per pixel, two groups of views
-    (200_011, (257, 131), 5, 4, True, 0, False),     # normal test and radius rule: the record carries the layer count
-    (200_011, (257, 131), 4, 5, True, 1, False),     # dropped points stay in the stream for the visible list
-    (60_000, (64, 48), 2, 5, True, 0, False),        # a tiny image: positions on both sides
-    (150_000, (256, 128), 2, 5, True, 0, True),      # drop-out decisions from the caller's mask
+@pytest.mark.parametrize("points,size,views,layers,rule,ghost,mask,model,streams", [
+    # the library keeps to the positions on both sides
+    (1, (40, 24), 1, 1, False, 0, False, "pinhole", False),           # one point, one layer
+    (257, (33, 17), 3, 3, False, 0, False, "pinhole", False),         # one point past a chunk, odd planes
+    (90_011, (101, 57), 5, 4, False, 0, False, "pinhole", False),     # two groups of views
+    (60_000, (64, 48), 2, 5, True, 0, False, "pinhole", False),       # normal test and radius rule
+    (150_000, (256, 128), 2, 5, True, 0, True, "pinhole", False),     # drop-out decisions from the caller's mask
+    (200_011, (257, 131), 4, 5, True, 1, False, "pinhole", False),    # dropped points are listed
+    # streams on one side
+    (300_033, (101, 57), 5, 4, False, 0, False, "pinhole", True),     # a tiny coarsest layer: layer by layer; the fifth view goes without
+    (300_033, (101, 57), 3, 1, False, 0, False, "pinhole", True),     # one layer of 5757 pixels: all reads first
+    (560_000, (201, 112), 4, 2, False, 1, True, "pinhole", True),     # two layers, dropped points stay in the stream
+    (257, (13, 9), 1, 2, True, 0, False, "pinhole", True),            # normal test and radius rule: the record carries the layer count
+    (200_011, (257, 131), 5, 4, True, 0, False, "pinhole", True),     # a group of four on positions, the fifth view with streams
+    (800_001, (97, 61), 4, 5, True, 1, False, "pinhole", True),       # dropped points stay in the stream for the visible list
+    (760_000, (64, 48), 2, 5, True, 0, True, "pinhole", True),        # drop-out decisions from the caller's mask
+    (1, (40, 24), 1, 1, False, 0, False, "ocam", True),               # one record, every other segment empty
+    (255, (33, 17), 3, 3, False, 0, False, "ocam", True),
+    (257, (33, 17), 5, 2, False, 0, False, "ocam", True),             # one point past a chunk, two groups
+    (70_001, (101, 57), 5, 4, False, 1, False, "ocam", True),
+    (70_001, (161, 97), 1, 3, True, 0, False, "ocam", True),          # normal test and radius rule
 ])
-def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib, points, size, views, layers, rule, ghost, mask):
+def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib, points, size, views, layers, rule, ghost, mask, model, streams):
     """Full workspace (the prepass drops points that already fail the depth test everywhere) against the small one (every
-    point is projected and tested again): the same depths, weights and listed points bit for bit."""
+    point is projected and tested again): the same depths, weights and listed points bit for bit. streams: what the library does
+    with the full workspace."""
     rng = np.random.default_rng(points + layers)
-    cfg = synth.make_config("c2", n_points=points, n_views=views, size=size, layers=layers)
+    cfg = synth.make_config("c2" if model == "pinhole" else "c3", n_points=points, n_views=views, size=size, layers=layers)
     a, params = cfg["arrays"], cfg["params"]
     params.dropout, params.dropout_seed, params.ghost_gradients = 0.3, 17, ghost
+    if model == "ocam":
+        a["poses"] = np.stack([synth.look_at_pose((0.1 * k, 0, 0), (0.3 * k, 0.2, 4), (0, -1, 0.01)) for k in range(views)])
+        cfg["views"] = [dict(cfg["views"][0], image_index=k) for k in range(views)]
     if rule:
         nrm = rng.normal(size=(points, 3))
         nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
@@ -400,6 +419,9 @@ def test_candidate_streams_leave_out_only_what_the_blend_kernel_refuses(cuda_lib
         params.check_normal = params.drop_out_points_by_radius = 1
     scene = to_scene(a)
     dm = torch.from_numpy(rng.integers(0, 2, (views, points)).astype(np.uint8)).cuda() if mask else None
+    sc, va = fill_scene_struct(scene.tensors(), lambda t: t.data_ptr()), capi.make_views(cfg["views"])
+    used = cuda_lib.adop_raster_forward_workspace_bytes(ctypes.byref(sc), va, views, ctypes.byref(params), layers)
+    assert (used == cuda_lib.adop_raster_workspace_bytes_full(points, views, *size, layers, 4)) == streams
     out = []
     for full in (False, True):
         fwd = PointRasterizer("cuda:0", full_workspace=full).forward(scene, cfg["views"], params, layers, dropout_mask=dm)
