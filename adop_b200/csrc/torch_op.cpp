@@ -137,37 +137,36 @@ static adop_scene make_scene(RenderInfo& info, const Tensor& texture, const Tens
 
 // Returns the size the library is told (it picks its kernels by it), which may be less than what an earlier call left behind.
 static size_t ensure_workspace(RenderInfo& info, const std::vector<adop_view>& views, int64_t num_layers, const adop_scene& sc,
-                               const torch::TensorOptions& opt, bool forward)
+                               const adop_render_params& params, const torch::TensorOptions& opt, bool forward)
 {
-    // With the full workspace the depth prepass hands the points that can still be accepted to the blend kernel
-    // (adop_raster_workspace_bytes_full); where the device has no room for it, the small one does.
-    size_t need = adop_raster_workspace_bytes(views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
-    TORCH_CHECK(need > 0, "invalid view size / layer count");
+    const size_t small = adop_raster_workspace_bytes(views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
+    TORCH_CHECK(small > 0, "invalid view size / layer count");
     auto provide = [&](size_t bytes)
     {
         if (!info.workspace.defined() || (size_t)info.workspace.numel() < bytes) info.workspace = torch::empty({(int64_t)bytes}, opt.dtype(torch::kUInt8));
+        return bytes;
     };
-    bool full = forward;
-    if (full)
+    // a forward call takes what it makes use of, or the small size where the device has no room for that (0: the arguments
+    // are refused, which the call itself reports)
+    const size_t used = forward ? adop_raster_forward_workspace_bytes(&sc, views.data(), (int32_t)views.size(), &params, (int32_t)num_layers) : 0;
+    size_t told = 0;
+    if (used > small)
     {
-        const size_t bytes = adop_raster_workspace_bytes_full(sc.num_points, (int32_t)views.size(), views[0].w, views[0].h, (int32_t)num_layers, sc.channels);
         try
         {
-            provide(bytes);
-            need = bytes;
+            told = provide(used);
         }
         catch (const c10::OutOfMemoryError&)
         {
-            full = false;
         }
     }
-    if (!full) provide(need);
+    if (told == 0) told = provide(small);
     if (!info.texture_interleaved.defined() || info.texture_interleaved.size(0) != sc.num_texels || info.texture_interleaved.size(1) != sc.channels)
     {
         info.texture_interleaved = torch::empty({sc.num_texels, sc.channels}, opt);
         info.grad_texture_interleaved = torch::empty({sc.num_texels, sc.channels}, opt);
     }
-    return need;
+    return told;
 }
 
 // What a forward call used and its backward call must use again, whatever happens to the RenderInfo in between (a second
@@ -207,7 +206,7 @@ struct PointRender : public torch::autograd::Function<PointRender>
         }
         const int B = (int)info->images.size(), L = (int)info->num_layers, C = sc.channels;
         auto opt = texture.options();
-        const size_t workspace_bytes = ensure_workspace(*info, info->images, info->num_layers, sc, opt, true);
+        const size_t workspace_bytes = ensure_workspace(*info, info->images, info->num_layers, sc, info->params, opt, true);
         check_status(adop_texture_interleave(sc.texture, info->texture_interleaved.data_ptr<float>(), C, sc.num_texels, stream),
                      "adop_texture_interleave");
         sc.texture_interleaved = info->texture_interleaved.data_ptr<float>();
@@ -286,7 +285,7 @@ struct PointRender : public torch::autograd::Function<PointRender>
         if (has(env_map)) call.env_map = env_map;
         adop_scene sc = make_scene(call, texture, background, points, intrinsics);
         // the shared [T,C] working copy may belong to a later forward call by now: rebuild it from this call's descriptors
-        const size_t workspace_bytes = ensure_workspace(*info, views, L, sc, texture.options(), false);
+        const size_t workspace_bytes = ensure_workspace(*info, views, L, sc, params, texture.options(), false);
         check_status(adop_texture_interleave(sc.texture, info->texture_interleaved.data_ptr<float>(), sc.channels, sc.num_texels, stream),
                      "adop_texture_interleave");
         sc.texture_interleaved = info->texture_interleaved.data_ptr<float>();

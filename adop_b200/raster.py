@@ -122,10 +122,9 @@ class PointRasterizer:
     """Owns the reusable scratch (the role of PointRendererCache, PointRenderer.h:96-157)."""
 
     def __init__(self, device="cuda:0", interleave_descriptors=True, full_workspace=None):
-        """full_workspace: True sizes the forward scratch with adop_raster_workspace_bytes_full (16 bytes per point and view
-        of a group more), which lets the depth prepass hand the projected points that can still be accepted to the blend
-        kernel instead of the blend kernel reading the cloud and projecting again; False keeps the small workspace. None
-        (default): the full workspace, or the small one where the device has no room for it."""
+        """full_workspace: None (default) sizes the forward scratch with adop_raster_forward_workspace_bytes, by what the call
+        makes use of (candidate streams, 16 bytes per point and view of a group, only where it has any), or small where the
+        device has no room for that; True with adop_raster_workspace_bytes_full, False always small."""
         self.lib = capi.load_library()
         self.device = torch.device(device)
         self._ws = None
@@ -156,12 +155,26 @@ class PointRasterizer:
             need = self.lib.adop_raster_workspace_bytes(w, h, layers, channels)
         if need == 0:
             raise ValueError("invalid size")
+        return self._reserve(need)
+
+    def _reserve(self, need):
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
         # the library picks its kernels by the size it is told: it is told the size asked for, not what an earlier, larger
         # call left behind
         self._ws_bytes = need
         return self._ws
+
+    def _forward_workspace(self, sc, va, params, num_layers):
+        w, h = va[0].w, va[0].h
+        if self.full_workspace is None:
+            need = self.lib.adop_raster_forward_workspace_bytes(C.byref(sc), va, len(va), C.byref(params), num_layers)
+            if need > 0:  # 0: the arguments are refused, which the forward call reports
+                try:
+                    return self._reserve(need)
+                except torch.cuda.OutOfMemoryError:
+                    pass
+        return self._workspace(w, h, num_layers, sc.channels, sc.num_points, len(va), full=bool(self.full_workspace))
 
     def forward(self, scene, views, params, num_layers, dropout_mask=None, out=None, record_visible=True,
                 refresh_descriptors=True, packed_depth=False, touched=None):
@@ -179,13 +192,7 @@ class PointRasterizer:
             # rendering frame after frame), so the [T,C] working copy is reused as it is
             sc = self._scene_struct(scene, refresh=refresh_descriptors)
             ch = sc.channels
-            if self.full_workspace is None:
-                try:
-                    ws = self._workspace(w, h, num_layers, ch, sc.num_points, B, full=True)
-                except torch.cuda.OutOfMemoryError:
-                    ws = self._workspace(w, h, num_layers, ch)
-            else:
-                ws = self._workspace(w, h, num_layers, ch, sc.num_points, B, full=bool(self.full_workspace))
+            ws = self._forward_workspace(sc, va, params, num_layers)
             sizes = capi.layer_sizes(w, h, num_layers)
             if out is None:
                 f32 = dict(dtype=torch.float32, device=self.device)

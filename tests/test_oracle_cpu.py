@@ -495,16 +495,20 @@ def test_c_abi_library_exports_every_declared_symbol():
     assert lib.adop_raster_workspace_bytes(0, 1080, 4, 4) == 0
 
 
-def _forward_workspace(points, size, views, layers=4, channels=4, model=0, rule=False, normals=False):
-    """(what a forward pass of these arguments makes use of, small size, full size); nothing is read on a device."""
-    lib = capi.load_library()
+def _forward_arguments(points, size, views, channels=4, model=0, rule=False, normals=False):
     sc, params = capi.AdopScene(), capi.default_render_params()
     sc.num_points = sc.num_texels = points
     sc.channels, sc.num_images, sc.num_cameras, sc.intrinsics_cols = channels, 1, 1, 13
-    sc.position = sc.texture = sc.background = sc.poses = sc.intrinsics = 4096  # any address
+    sc.position = sc.texture = sc.background = sc.poses = sc.intrinsics = 4096  # any address: nothing is read
     sc.normal = 4096 if normals else None
     params.drop_out_points_by_radius = int(rule)
-    va = capi.make_views([dict(w=size[0], h=size[1], image_index=0, camera_model=model)] * views)
+    return sc, capi.make_views([dict(w=size[0], h=size[1], image_index=0, camera_model=model)] * views), params
+
+
+def _forward_workspace(points, size, views, layers=4, channels=4, model=0, rule=False, normals=False):
+    """(what a forward pass of these arguments makes use of, small size, full size); nothing is read on a device."""
+    lib = capi.load_library()
+    sc, va, params = _forward_arguments(points, size, views, channels, model, rule, normals)
     used = lib.adop_raster_forward_workspace_bytes(ctypes.byref(sc), va, views, ctypes.byref(params), layers)
     return (used, lib.adop_raster_workspace_bytes(*size, layers, channels),
             lib.adop_raster_workspace_bytes_full(points, views, *size, layers, channels))
@@ -539,6 +543,27 @@ def test_forward_workspace_without_streams_holds_the_group_accumulators_only():
     lib = capi.load_library()
     assert lib.adop_raster_forward_workspace_bytes(None, None, 1, None, 4) == 0
     assert _forward_workspace(1000, (4, 4), 1, layers=4)[0] == 0  # the coarsest layer would be empty
+
+
+@pytest.mark.parametrize("points,size,views,kw", [
+    (10_000_000, (1920, 1080), 16, {}),            # a training batch that keeps to its positions
+    (40_000_000, (1280, 720), 1, {}),              # a viewer frame that does
+    (500_000, (512, 512), 4, {}),                  # accumulators of a group
+    (200_000, (320, 240), 3, dict(model=1)),       # candidate streams
+])
+def test_rasterizer_takes_the_workspace_that_the_call_reads(points, size, views, kw):
+    """The scratch of a forward call is what the library makes use of, not room for streams that the call would not write."""
+    from adop_b200.raster import PointRasterizer
+    used, small, full = _forward_workspace(points, size, views, **kw)
+    sc, va, params = _forward_arguments(points, size, views, **kw)
+    r = PointRasterizer("cpu")  # the scratch alone: nothing is launched
+    ws = r._forward_workspace(sc, va, params, 4)
+    assert ws.numel() == r._ws_bytes == used
+    assert (used == full) == bool(kw) and (kw or used <= small + 256 + (24 << 20))
+    for option, size_of in ((True, full), (False, small)):
+        r = PointRasterizer("cpu", full_workspace=option)
+        r._forward_workspace(sc, va, params, 4)
+        assert r._ws_bytes == size_of
 
 
 def test_struct_sizes_match_the_header():

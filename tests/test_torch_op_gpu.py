@@ -229,3 +229,23 @@ def test_outlier_cloud_through_the_operator(oracle, cuda_lib, op):
     _close(points.grad, ref_b["points"], "grad points")
     _close(tangents.grad, ref_b["pose"], "grad pose")
     _close(intrinsics.grad, ref_b["intrinsics"], "grad intrinsics")
+
+
+def test_operator_takes_the_workspace_that_the_call_reads(cuda_lib, op):
+    """What a RenderInfo keeps after a plain single view: the small scratch and the two [T,C] copies, no room for candidate
+    streams (16 bytes per point more, 72 MB here), which such a call does not write."""
+    n = 4_000_000
+    cfg = synth.make_config("c2", n_points=n, n_views=1, size=(64, 48), sort=False)
+    a = cfg["arrays"]
+    dev = torch.device("cuda:0")
+    t = {k: torch.from_numpy(a[k]).to(dev) for k in ("texture", "background", "position", "intrinsics")}
+    tangents = torch.zeros((1, 6), dtype=torch.float64, device=dev)
+    info = _info(cfg, dev)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    out = op.blend_point_cloud(t["texture"], t["background"], t["position"], tangents, t["intrinsics"], info)
+    torch.cuda.synchronize()
+    del out
+    kept = torch.cuda.memory_allocated() - before
+    copies = 2 * 4 * 4 * n
+    assert copies < kept < copies + cuda_lib.adop_raster_workspace_bytes(64, 48, 4, 4) + (8 << 20)
