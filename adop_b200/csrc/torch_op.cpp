@@ -39,6 +39,7 @@ struct RenderInfo : torch::CustomClassHolder
     int64_t num_layers = 1;
     // reusable buffers (the role of PointRendererCache, PointRenderer.h:96-157)
     Tensor workspace, texture_interleaved, grad_texture_interleaved;
+    size_t refused_bytes = ~(size_t)0;  // the smallest workspace that the device had no room for
 
     RenderInfo() { adop_render_params_default(&params); }
 
@@ -150,7 +151,7 @@ static size_t ensure_workspace(RenderInfo& info, const std::vector<adop_view>& v
     // are refused, which the call itself reports)
     const size_t used = forward ? adop_raster_forward_workspace_bytes(&sc, views.data(), (int32_t)views.size(), &params, (int32_t)num_layers) : 0;
     size_t told = 0;
-    if (used > small)
+    if (used > small && used < info.refused_bytes)
     {
         try
         {
@@ -158,6 +159,7 @@ static size_t ensure_workspace(RenderInfo& info, const std::vector<adop_view>& v
         }
         catch (const c10::OutOfMemoryError&)
         {
+            info.refused_bytes = used;  // not asked for again: every refusal costs a synchronisation and the allocator's cached blocks
         }
     }
     if (told == 0) told = provide(small);

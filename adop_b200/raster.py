@@ -128,6 +128,7 @@ class PointRasterizer:
         self.lib = capi.load_library()
         self.device = torch.device(device)
         self._ws = None
+        self._refused_bytes = float("inf")  # the smallest scratch that the device had no room for
         self.interleave_descriptors = interleave_descriptors
         self.full_workspace = full_workspace
         self._tex_i = None    # [T,C] working copy of the descriptors, refreshed by every forward call
@@ -169,11 +170,12 @@ class PointRasterizer:
         w, h = va[0].w, va[0].h
         if self.full_workspace is None:
             need = self.lib.adop_raster_forward_workspace_bytes(C.byref(sc), va, len(va), C.byref(params), num_layers)
-            if need > 0:  # 0: the arguments are refused, which the forward call reports
+            if 0 < need < self._refused_bytes:  # 0: the arguments are refused, which the forward call reports
                 try:
                     return self._reserve(need)
                 except torch.cuda.OutOfMemoryError:
-                    pass
+                    # not asked for again: every refusal costs a synchronisation and the allocator's cached blocks
+                    self._refused_bytes = need
         return self._workspace(w, h, num_layers, sc.channels, sc.num_points, len(va), full=bool(self.full_workspace))
 
     def forward(self, scene, views, params, num_layers, dropout_mask=None, out=None, record_visible=True,

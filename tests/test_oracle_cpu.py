@@ -566,6 +566,31 @@ def test_rasterizer_takes_the_workspace_that_the_call_reads(points, size, views,
         assert r._ws_bytes == size_of
 
 
+def test_rasterizer_asks_once_for_a_workspace_that_is_refused(monkeypatch):
+    """Where the device has no room for the candidate streams the small scratch does, and the refused size is not asked for
+    again (a refusal makes the caching allocator synchronise and give back its blocks); smaller ones still are."""
+    from adop_b200.raster import PointRasterizer
+    asked, empty = [], torch.empty
+
+    def limited(size, *a, **k):
+        asked.append(size)
+        if size > 64 << 20:
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return empty(size, *a, **k)
+
+    monkeypatch.setattr(torch, "empty", limited)
+    r = PointRasterizer("cpu")
+    large, medium = (4_000_000, (320, 240), 4), (300_000, (320, 240), 4)
+    for _ in range(3):
+        sc, va, params = _forward_arguments(*large, model=1)
+        ws = r._forward_workspace(sc, va, params, 4)
+        assert ws.numel() == r._ws_bytes == _forward_workspace(*large, model=1)[1]
+    assert asked == [_forward_workspace(*large, model=1)[2], _forward_workspace(*large, model=1)[1]]
+    sc, va, params = _forward_arguments(*medium, model=1)
+    r._forward_workspace(sc, va, params, 4)
+    assert r._ws_bytes == asked[-1] == _forward_workspace(*medium, model=1)[2]
+
+
 def test_struct_sizes_match_the_header():
     """ctypes mirrors must have the C layout (compiled probe with the system compiler)."""
     import subprocess

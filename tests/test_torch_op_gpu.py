@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from adop_b200 import build, synth
+from adop_b200.raster import PointRasterizer, Scene
 
 pytestmark = pytest.mark.gpu
 
@@ -249,3 +250,46 @@ def test_operator_takes_the_workspace_that_the_call_reads(cuda_lib, op):
     kept = torch.cuda.memory_allocated() - before
     copies = 2 * 4 * 4 * n
     assert copies < kept < copies + cuda_lib.adop_raster_workspace_bytes(64, 48, 4, 4) + (8 << 20)
+
+
+def test_a_workspace_that_is_refused_is_asked_for_once(cuda_lib, op):
+    """A limit on the allocator leaves no room for the candidate streams: the operator and the rasterizer go on with the small
+    scratch, same results, and do not ask again (each refusal would make the allocator give back its cached blocks)."""
+    n = 2_000_000
+    cfg = synth.make_config("c3", n_points=n, size=(32, 16), sort=False)  # one screen tile: the list takes less than the streams
+    a = cfg["arrays"]
+    dev = torch.device("cuda:0")
+    t = {k: torch.from_numpy(a[k]).to(dev) for k in ("texture", "background", "position", "intrinsics")}
+    tangents = torch.zeros((1, 6), dtype=torch.float64, device=dev)
+    scene = Scene(t["position"], t["texture"], t["background"], torch.from_numpy(a["poses"]).to(dev), t["intrinsics"])
+    args = (t["texture"], t["background"], t["position"], tangents, t["intrinsics"])
+    omni = cfg["views"]
+    pinhole = [dict(omni[0], camera_model=0)]  # (no streams)
+    expect = PointRasterizer(dev).forward(scene, omni, cfg["params"], 4)
+    limited, info = PointRasterizer(dev), _info(dict(cfg, views=pinhole), dev)
+    # everything but the streams is there already: layers, list and copies of the rasterizer, the operator's copies, and a cached
+    # block of its list's size
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    out = limited.forward(scene, pinhole, cfg["params"], 4)
+    colors = op.blend_point_cloud(*args, info)
+    del colors
+    torch.cuda.synchronize()
+    rows = torch.tensor([[32, 16, 0, 0, omni[0]["camera_model"]]]), torch.tensor([[1.0, 1.0, 0.0, 0.0, 0.0]])
+    info.set_views(*rows)
+    ooms = torch.cuda.memory_stats(dev)["num_ooms"]
+    try:
+        torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved(dev) / torch.cuda.get_device_properties(dev).total_memory, dev)
+        for _ in range(3):
+            limited.forward(scene, omni, cfg["params"], 4, out=out)
+        assert torch.cuda.memory_stats(dev)["num_ooms"] == ooms + 1
+        for _ in range(3):
+            colors = None
+            colors = op.blend_point_cloud(*args, info)
+        assert torch.cuda.memory_stats(dev)["num_ooms"] == ooms + 2
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+    for l in range(4):
+        assert torch.equal(out.depths[l], expect.depths[l]) and torch.equal(out.weights[l], expect.weights[l])
+        _close(out.colors[l], expect.colors[l].cpu().numpy(), f"small scratch colour {l}")
+        _close(colors[l], expect.colors[l].cpu().numpy(), f"operator colour {l}")
