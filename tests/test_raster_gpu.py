@@ -475,6 +475,38 @@ def test_batch_of_both_camera_models_equals_its_views_one_by_one(cuda_lib):
     assert int((batch["count_pose"] > 0).sum()) == 6 and bool((batch["count_intrinsics"] > 0).all())
 
 
+def test_pose_gradient_of_a_batch_is_summed_in_double(cuda_lib):
+    """Every term of the x translation's gradient is the same float32 number, so its exact sum is known and what is measured is the
+    summation alone: points at distance 1 on every third pixel (their stencil sees uncovered neighbours), 60 per pixel, sixteen
+    views in one launch. 350 terms per lane in float32 are 4.5e-6 off; 16 terms and a warp's five additions round 21 times, each by
+    2^-24 of the sum at most."""
+    w, h, views, stack, f = 640, 480, 16, 60, 256.0
+    px, py = np.meshgrid(np.arange(4, w - 4, 3), np.arange(4, h - 4, 3))  # 1 modulo 3: the right neighbour is 2 modulo 3
+    n = px.size * stack
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, 0] = np.repeat((px.ravel() - w / 2) / f, stack)
+    pos[:, 1] = np.repeat((py.ravel() - h / 2) / f, stack)
+    pos[:, 2] = 1.0
+    term = 1.1396560668945312
+    tex = np.zeros((4, n), np.float32)
+    tex[0] = term / 32  # 256 (focal length) / 2 (central difference) / 4 (channels) = 32
+    intr = np.zeros((1, 13), np.float32)
+    intr[0, :4] = f, f, w / 2, h / 2
+    poses = np.tile(np.array([0, 0, 0, 1, 0, 0, 0, 0], np.float64), (views, 1))
+    scene = to_scene(dict(position=pos, texture=tex, background=np.zeros(4, np.float32), poses=poses, intrinsics=intr, env_map=None))
+    params = capi.default_render_params()
+    params.dropout, params.check_normal, params.drop_out_points_by_radius, params.dist_cutoff = 0.0, 0, 0, 100.0
+    r = PointRasterizer("cuda:0")
+    fwd = r.forward(scene, [dict(w=w, h=h, image_index=k) for k in range(views)], params, 1)
+    assert not bool(fwd.list_unusable().any())
+    grad = torch.zeros((views, 4, h, w), device="cuda:0")
+    grad[:, 0, :, 2::3] = 1.0
+    g = r.backward(scene, params, fwd, [grad], normalize=False)
+    assert bool((g["count_pose"] == n).all())
+    off = (g["pose"][:, 0].cpu().numpy() / (n * term) - 1).astype(np.float64)
+    assert np.abs(off).max() <= 21 * 2.0 ** -24, off
+
+
 def test_backward_mode_4(oracle, cuda_lib):
     cfg = synth.make_config("c1", n_points=40_000, size=(96, 96))
     cfg["params"].test_backward_mode = 4
