@@ -15,10 +15,6 @@
 //    are reduced warp -> block in shared memory and leave as one atomic per component and block;
 //  * the all-points kernels read the ghost stencil from one interleaved record per pixel [I_0..I_C-1, G_0..G_C-1] that a
 //    preparation pass builds (a neighbour then costs one or two 32-byte sectors instead of 2C).
-#include <cooperative_groups.h>
-
-#include <algorithm>
-
 #include "common.cuh"
 
 namespace adop {
@@ -211,17 +207,16 @@ struct BackwardTargets
     float* count_intrinsics;  // element of this view's camera
 };
 
-// interleaved [I | G] of a pyramid pixel, written by the preparation pass (in the same launch where that serves several
-// views: no read-only loads)
+// interleaved [I | G] of a pyramid pixel, written by the preparation pass
 template <int C>
-__device__ __forceinline__ void load_record(const float* records, size_t r, float* out)
+__device__ __forceinline__ void load_record(const float* __restrict__ records, size_t r, float* out)
 {
     constexpr int RB = (2 * C + 3) & ~3;
     const float4* src = reinterpret_cast<const float4*>(records + r * RB);
 #pragma unroll
     for (int k = 0; k < RB / 4; ++k)
     {
-        float4 a = src[k];
+        float4 a = __ldg(src + k);
         out[4 * k] = a.x; out[4 * k + 1] = a.y; out[4 * k + 2] = a.z; out[4 * k + 3] = a.w;
     }
 }
@@ -386,7 +381,8 @@ __device__ __forceinline__ void geo_block_reduce(GeoShared<MODEL>* s, const GeoA
 
 // K5 (all points): the reference's structure, one thread per point walking its layers (RenderBackward, :396-724). Used
 // when the forward pass recorded no visible list (or a tile's bucket overflowed, or the list was used before).
-template <int C, int MODEL>
+// records: [I | G] of every pixel from a launch of the preparation pass; null: the same values from the planes.
+template <int C, int MODEL, bool RECORDS>
 __device__ __forceinline__ void splat_backward_part(const PointStreams& pts, const ViewCam& cam, const KernelParams& kp, const LayerTable& lt, int view,
                                                     const BackwardTargets& bt, const float* records, int image, int camera, int intrinsics_cols)
 {
@@ -432,7 +428,12 @@ __device__ __forceinline__ void splat_backward_part(const PointStreams& pts, con
                 if (bt.grad_texture)
                 {
                     float rc[RB];
-                    load_record<C>(records, rbase, rc);
+                    if (RECORDS) load_record<C>(records, rbase, rc);
+                    else
+                    {
+#pragma unroll
+                        for (int c = 0; c < C; ++c) rc[C + c] = __ldg(view_grad<C>(lt, l, view) + (size_t)c * w * h + pix);
+                    }
                     const float iw = 1.f / wgt;
 #pragma unroll
                     for (int c = 0; c < C; ++c) dg[c] += iw * rc[C + c];
@@ -450,7 +451,20 @@ __device__ __forceinline__ void splat_backward_part(const PointStreams& pts, con
             const size_t nb[4] = {pix - 1, pix + 1, pix - (size_t)w, pix + (size_t)w};
             float rn[4][RB];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) load_record<C>(records, (size_t)lt.rec_off[l] + nb[k], rn[k]);
+            for (int k = 0; k < 4; ++k)
+            {
+                if (RECORDS) load_record<C>(records, (size_t)lt.rec_off[l] + nb[k], rn[k]);
+                else
+                {
+                    const bool covered = __ldg(W + nb[k]) != 0.f;
+#pragma unroll
+                    for (int c = 0; c < C; ++c)
+                    {
+                        rn[k][c] = covered ? __ldg(view_color<C>(lt, l, view) + (size_t)c * w * h + nb[k]) : __ldg(bt.background + c);
+                        rn[k][C + c] = __ldg(view_grad<C>(lt, l, view) + (size_t)c * w * h + nb[k]);
+                    }
+                }
+            }
             V2 g = stencil_gradient<C>(kp, T_p, rn, q.z, W, D, nb);
             chain_gradient<MODEL>(cam, kp, f, g, scale, gp, acc);
         }
@@ -467,32 +481,7 @@ template <int C, int MODEL>
 __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts, const ViewCam* __restrict__ camp, const ViewRows* __restrict__ rows,
                                                                 KernelParams kp, LayerTable lt, BackwardTargets bt, const float* records, int intrinsics_cols)
 {
-    splat_backward_part<C, MODEL>(pts, *camp, kp, lt, 0, bt, records, rows->image, rows->camera, intrinsics_cols);
-}
-
-// Behind the visible lists: the last kernel of the pass, one cooperative launch for all its views. A view that ran on its list
-// only has the list marked as consumed when its entries were turned into work items; a view whose list was not usable gets
-// the two all-points steps here. Nearly always there is nothing to do, and a launch per view and step for nothing was
-// 32 of the 130 launches of a 16-view training step.
-template <int C, int MODEL>
-__global__ void __launch_bounds__(kBlock) k_behind_lists(PointStreams pts, const ViewCam* __restrict__ cams, const ViewRows* __restrict__ rows, KernelParams kp,
-                                                          LayerTable lt, BackwardTargets bt, float* records, int intrinsics_cols, ViewLists lists, HoleArgs ha,
-                                                          int views, int mark_consumed)
-{
-    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    for (int view = 0; view < views; ++view)
-    {
-        int* header = list_of_view(lists.first, lists.view_ints, view).header;
-        if (__ldg(header + kListGo) != 0)  // the same in every block: written by an earlier kernel
-        {
-            if (mark_consumed && blockIdx.x == 0 && threadIdx.x == 0) header[kListConsumed] = 1;
-            continue;
-        }
-        prepare_backward_part<C>(lt, view, cams[view], kp, bt.background, records, ha);
-        grid.sync();
-        splat_backward_part<C, MODEL>(pts, cams[view], kp, lt, view, bt, records, rows[view].image, rows[view].camera, intrinsics_cols);
-        grid.sync();  // the next view rewrites the records
-    }
+    splat_backward_part<C, MODEL, true>(pts, *camp, kp, lt, 0, bt, records, rows->image, rows->camera, intrinsics_cols);
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -1144,6 +1133,51 @@ __global__ void __launch_bounds__(kBlock, MODEL == kPinholeDistortion ? 4 : 3)
         hole_gradients_part<C>(lt, view, cams + view, kp, ha, (int)blockIdx.x - chain_blocks, (int)gridDim.x - chain_blocks);
 }
 
+// Behind the visible lists: the end of the pass. A view that ran on its list only has the list marked as consumed when its
+// entries were turned into work items; for a view whose list was not usable the whole launch walks all points. Nearly always
+// there is nothing to do, and a launch per view and step for nothing was 32 of the 130 launches of a 16-view training step; but
+// no block may wait for another one either (a launch whose blocks do has to fit the GPU at once, which a part of it, an MPS
+// share or a green context, refuses). So
+//  * up to four channels (kBehindFromPlanes) everything is one launch for all views, which takes pixels and holes straight
+//    from the planes: they fit L2, and 16 views of 10 M points at 1080p take 13.3 ms (15.3 ms from records);
+//  * with more channels they do not fit, and a visit would fetch 54 sectors instead of 10 (two views of 3 M points at 1080p,
+//    16 channels: 2.8 ms, from records 1.9 ms). There a launch that prepares the records goes before, and as many views share
+//    the two as the workspace has room for records.
+template <int C> constexpr bool kBehindFromPlanes = C <= 4;
+struct RecordSpace
+{
+    float* first;        // records of the launch's first view
+    size_t view_floats;  // distance from view to view
+};
+template <int C>
+__global__ void __launch_bounds__(kBlock) k_prepare_behind_lists(LayerTable lt, const ViewCam* __restrict__ cams, KernelParams kp, const float* __restrict__ background,
+                                                                  ViewLists lists, RecordSpace records, HoleArgs ha)
+{
+    const int view = (int)blockIdx.y;
+    if (__ldg(list_of_view(lists.first, lists.view_ints, view).header + kListGo) != 0) return;
+    prepare_backward_part<C>(lt, view, cams[view], kp, background, records.first + view * records.view_floats, ha);
+}
+template <int C, int MODEL>
+__global__ void __launch_bounds__(kBlock) k_behind_lists(PointStreams pts, const ViewCam* __restrict__ cams, const ViewRows* __restrict__ rows, KernelParams kp,
+                                                          LayerTable lt, BackwardTargets bt, int intrinsics_cols, ViewLists lists, RecordSpace records, HoleArgs ha,
+                                                          int views, int mark_consumed)
+{
+    for (int view = 0; view < views; ++view)
+    {
+        int* header = list_of_view(lists.first, lists.view_ints, view).header;
+        if (__ldg(header + kListGo) != 0)  // the same in every block: written by an earlier kernel
+        {
+            if (mark_consumed && blockIdx.x == 0 && threadIdx.x == 0) header[kListConsumed] = 1;
+            continue;
+        }
+        if (kBehindFromPlanes<C> && (ha.grad_background || ha.grad_env))
+            hole_gradients_part<C>(lt, view, cams + view, kp, ha, (int)blockIdx.x, (int)gridDim.x);
+        splat_backward_part<C, MODEL, !kBehindFromPlanes<C>>(pts, cams[view], kp, lt, view, bt, records.first + view * records.view_floats, rows[view].image,
+                                                             rows[view].camera, intrinsics_cols);
+        __syncthreads();  // the next view starts its block sums anew
+    }
+}
+
 // ------------------------------------------------------------------------------------------------------
 // NormalizeGradient, PointRenderer.cu:1534-1547
 __global__ void k_normalize_points(float4* g, int n)
@@ -1183,11 +1217,11 @@ static int blocks_per_view(int resident, int waves, int views, int most)
 }
 
 // The list kernels of `views` consecutive views of one camera model. lt, kp, cams, rows and lists are those of the first;
-// bt's pose and intrinsics rows are the tensors' first rows.
+// bt's pose and intrinsics rows are the tensors' first rows; records: room for record_views views.
 template <int C, int MODEL>
 static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* cams, const ViewRows* rows, const KernelParams& kp, const LayerTable& lt,
-                                        const TileTable& tt, const BackwardTargets& bt, float* records, int intrinsics_cols, const HoleArgs& ha,
-                                        cudaStream_t st, const ViewLists& lists, int views)
+                                        const TileTable& tt, const BackwardTargets& bt, float* records, int record_views, int intrinsics_cols,
+                                        const HoleArgs& ha, cudaStream_t st, const ViewLists& lists, int views)
 {
     const int want_geo = (bt.grad_points || bt.grad_pose || bt.grad_intrinsics) ? 1 : 0;
     const size_t smem = tile_smem_bytes(C, lt.L);
@@ -1227,12 +1261,26 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
         ADOP_LAUNCH("k_chain_and_holes", st, (k_chain_and_holes<C, MODEL><<<dim3((unsigned)(chain_blocks + hole_blocks), (unsigned)views), kBlock, 0, st>>>(
                                                  pts, cams, rows, kp, lt, bt, intrinsics_cols, lists, tt, ha, chain_blocks)));
     }
-    // one block per SM: an empty launch costs by its block count, and a cooperative one has to fit beside other work
-    static const int g_behind = std::min(resident_grid(k_behind_lists<C, MODEL>, 1ll << 40), sm_count());
-    PointStreams a_pts = pts; const ViewCam* a_cams = cams; const ViewRows* a_rows = rows; KernelParams a_kp = kp; LayerTable a_lt = lt; BackwardTargets a_bt = bt;
-    ViewLists a_lists = lists; HoleArgs a_ha = ha; int a_geo = want_geo;
-    void* args[] = {&a_pts, &a_cams, &a_rows, &a_kp, &a_lt, &a_bt, &records, &intrinsics_cols, &a_lists, &a_ha, &views, &a_geo};
-    ADOP_LAUNCH("k_behind_lists", st, ADOP_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_behind_lists<C, MODEL>), dim3((unsigned)g_behind), dim3(kBlock), args, 0, st)));
+    static const int g_behind = resident_grid(k_behind_lists<C, MODEL>, 1ll << 40);
+    const int together = kBehindFromPlanes<C> ? views : record_views;
+    for (int v = 0; v < views; v += together)
+    {
+        const int n = views - v < together ? views - v : together;
+        const LayerTable ltv = layer_table_of_view(lt, C, v);
+        KernelParams kv = kp;
+        kv.batch_slot += v;
+        if (kv.dropout_mask) kv.dropout_mask += (size_t)v * pts.n;
+        ViewLists lv = lists;
+        lv.first = list_of_view(lists.first, lists.view_ints, v);
+        const RecordSpace rs = {records, (size_t)lt.rec_off[kMaxLayers] * backward_record_floats(C)};
+        if (!kBehindFromPlanes<C>)
+        {
+            static const int g_prepare = resident_grid(k_prepare_behind_lists<C>, 1ll << 40);
+            const dim3 grid((unsigned)blocks_per_view(g_prepare, 1, n, (int)((lt.rec_off[kMaxLayers] + kBlock - 1) / kBlock)), (unsigned)n);
+            ADOP_LAUNCH("k_prepare_behind_lists", st, (k_prepare_behind_lists<C><<<grid, kBlock, 0, st>>>(ltv, cams + v, kv, bt.background, lv, rs, ha)));
+        }
+        ADOP_LAUNCH("k_behind_lists", st, (k_behind_lists<C, MODEL><<<g_behind, kBlock, 0, st>>>(pts, cams + v, rows + v, kv, ltv, bt, intrinsics_cols, lv, rs, ha, n, want_geo)));
+    }
     ADOP_CUDA_TRY(cudaGetLastError());
     return ADOP_OK;
 }
@@ -1255,10 +1303,10 @@ static adop_status launch_all_points_backward(const PointStreams& pts, const Vie
 // `views` consecutive views of one camera model, with lists or without; the pointers are the first view's.
 template <int C, int MODEL>
 static adop_status launch_views_backward(const PointStreams& pts, const ViewCam* cams, const ViewRows* rows, const KernelParams& kp, const LayerTable& lt,
-                                         const TileTable& tt, const BackwardTargets& bt, float* records, int intrinsics_cols, const HoleArgs& ha,
-                                         cudaStream_t st, const ViewLists& lists, int views)
+                                         const TileTable& tt, const BackwardTargets& bt, float* records, int record_views, int intrinsics_cols,
+                                         const HoleArgs& ha, cudaStream_t st, const ViewLists& lists, int views)
 {
-    if (lists.first.header) return launch_list_backward<C, MODEL>(pts, cams, rows, kp, lt, tt, bt, records, intrinsics_cols, ha, st, lists, views);
+    if (lists.first.header) return launch_list_backward<C, MODEL>(pts, cams, rows, kp, lt, tt, bt, records, record_views, intrinsics_cols, ha, st, lists, views);
     for (int v = 0; v < views; ++v)
     {
         KernelParams kv = kp;
@@ -1365,7 +1413,11 @@ extern "C" adop_status adop_raster_backward(const adop_scene* s, const adop_view
     bt.count_pose = io->grad_pose ? io->count_pose : nullptr;
     bt.grad_intrinsics = io->grad_intrinsics;
     bt.count_intrinsics = io->grad_intrinsics ? io->count_intrinsics : nullptr;
+    // the workspace holds the records of one view at least
     float* records = reinterpret_cast<float*>(static_cast<char*>(io->workspace) + kCamRegionBytes);
+    const size_t record_bytes = (size_t)base.rec_off[kMaxLayers] * backward_record_floats(C) * sizeof(float);
+    const size_t record_room = (io->workspace_bytes - kCamRegionBytes) / record_bytes;
+    const int record_views = (int)(record_room < kCamChunk ? record_room : kCamChunk);
     for (int l = 0; l < L; ++l)
     {
         base.depth[l] = io->layers[l].depth;
@@ -1397,8 +1449,8 @@ extern "C" adop_status adop_raster_backward(const adop_scene* s, const adop_view
             const ViewRows* row = rows + (b - b0);
             adop_status r;
 #define ADOP_VIEWS_BACKWARD(CC)                                                                                                                      \
-    r = pinhole ? launch_views_backward<CC, kPinholeDistortion>(pts, cam, row, kp, lt, tiles, bt, records, cols, ha, st, lists, e - b)               \
-                : launch_views_backward<CC, kOcam>(pts, cam, row, kp, lt, tiles, bt, records, cols, ha, st, lists, e - b)
+    r = pinhole ? launch_views_backward<CC, kPinholeDistortion>(pts, cam, row, kp, lt, tiles, bt, records, record_views, cols, ha, st, lists, e - b)               \
+                : launch_views_backward<CC, kOcam>(pts, cam, row, kp, lt, tiles, bt, records, record_views, cols, ha, st, lists, e - b)
             switch (C)
             {
                 case 3: ADOP_VIEWS_BACKWARD(3); break;

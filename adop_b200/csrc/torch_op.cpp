@@ -287,7 +287,7 @@ struct PointRender : public torch::autograd::Function<PointRender>
         if (has(env_map)) call.env_map = env_map;
         adop_scene sc = make_scene(call, texture, background, points, intrinsics);
         // the shared [T,C] working copy may belong to a later forward call by now: rebuild it from this call's descriptors
-        const size_t workspace_bytes = ensure_workspace(*info, views, L, sc, params, texture.options(), false);
+        ensure_workspace(*info, views, L, sc, params, texture.options(), false);
         check_status(adop_texture_interleave(sc.texture, info->texture_interleaved.data_ptr<float>(), sc.channels, sc.num_texels, stream),
                      "adop_texture_interleave");
         sc.texture_interleaved = info->texture_interleaved.data_ptr<float>();
@@ -344,7 +344,7 @@ struct PointRender : public torch::autograd::Function<PointRender>
         io.accumulate = 0;
         io.normalize = 1;
         io.workspace = info->workspace.data_ptr();
-        io.workspace_bytes = workspace_bytes;
+        io.workspace_bytes = (size_t)info->workspace.numel();  // views whose list was not usable share launches where there is room
         check_status(adop_raster_backward(&sc, views.data(), B, &params, L, &io, stream), "adop_raster_backward");
         // {texture, background, points, pose tangents, intrinsics}, the environment map, and nothing for the info object
         // (PointRenderer.cu:1641-1643, RenderInfo.cpp:56)

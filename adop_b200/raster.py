@@ -280,7 +280,7 @@ class PointRasterizer:
             io.normalize = 1 if normalize else 0
             ws = self._workspace(va[0].w, va[0].h, L, sc.channels, sc.num_points, B)
             io.workspace = ws.data_ptr()
-            io.workspace_bytes = self._ws_bytes
+            io.workspace_bytes = ws.numel()  # views whose list was not usable share launches where there is room
             io.visible_list = fwd.visible.data_ptr() if fwd.visible is not None else None
             if out.get("texture_interleaved") is not None:
                 # the caller keeps the descriptor gradients in [T,C] layout (the block the GPUs exchange, dist.py)

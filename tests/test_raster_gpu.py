@@ -356,6 +356,54 @@ def test_second_backward_on_the_same_list(oracle, cuda_lib):
         close(second[k], first[k].cpu().numpy(), name=f"second backward {k}")
 
 
+@pytest.fixture
+def eight_sm_stream():
+    """A stream of a green context with eight of the GPU's SMs: what a process sees that shares the GPU by parts."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def call(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    torch.zeros(1, device="cuda:0")  # the device's primary context exists
+    dev = call(drv.cuDeviceGet(0))
+    sms = call(drv.cuDeviceGetDevResource(dev, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, count, _ = call(drv.cuDevSmResourceSplitByCount(1, sms, 0, 8))
+    assert count == 1 and 8 <= groups[0].sm.smCount < sms.sm.smCount // 2
+    ctx = call(drv.cuGreenCtxCreate(call(drv.cuDevResourceGenerateDesc([groups[0]], 1)), dev, drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM.value))
+    stream = call(drv.cuGreenCtxStreamCreate(ctx, drv.CUstream_flags.CU_STREAM_NON_BLOCKING.value, 0))
+    yield torch.cuda.ExternalStream(int(stream), device="cuda:0")
+    torch.cuda.synchronize()
+    call(drv.cuStreamDestroy(stream) + (None,))
+    call(drv.cuGreenCtxDestroy(ctx) + (None,))
+
+
+@pytest.mark.parametrize("channels,model", [(4, "c2"), (8, "c2"), (4, "c3")])
+def test_both_directions_run_on_a_part_of_the_gpu(cuda_lib, eight_sm_stream, channels, model):
+    """No launch asks for more SMs than its stream has: with lists, and again on the same lists (all points behind them), the
+    results are those of the whole GPU."""
+    cfg = synth.make_config(model, n_points=60_000, n_views=3 if model == "c2" else None, size=(150, 83), channels=channels)
+    scene, params, L = to_scene(cfg["arrays"]), cfg["params"], cfg["num_layers"]
+    grads = [torch.from_numpy(g).cuda() for g in synth.upstream_gradients(cfg["meta"], batch=len(cfg["views"]))]
+    mask = torch.from_numpy(np.random.default_rng(3).integers(0, 2, (len(cfg["views"]), 60_000)).astype(np.uint8)).cuda()
+    want = dict(want_env=model == "c2", dropout_mask=mask)
+    r = PointRasterizer("cuda:0")
+    fwd = r.forward(scene, cfg["views"], params, L, dropout_mask=mask)
+    whole = r.backward(scene, params, fwd, grads, **want)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(eight_sm_stream):
+        part = PointRasterizer("cuda:0")
+        f = part.forward(scene, cfg["views"], params, L, dropout_mask=mask)
+        first = part.backward(scene, params, f, grads, **want)
+        second = part.backward(scene, params, f, grads, **want)
+    torch.cuda.synchronize()
+    for l in range(L):
+        assert torch.equal(f.depths[l], fwd.depths[l]) and torch.equal(f.weights[l], fwd.weights[l])
+    for name, b in (("first", first), ("second", second)):
+        for k in ("texture", "background", "points", "pose", "intrinsics") + (("env_map",) if model == "c2" else ()):
+            close(b[k], whole[k].cpu().numpy(), name=f"eight SMs {name} {k}")
+
+
 def test_small_workspace_matches_full_workspace(cuda_lib):
     """With the full workspace the depth prepass hands projected points to the blend kernel; with the small one the blend
     kernel projects again. Same depth and weight bits, colours and gradients within the atomic-order tolerance."""
