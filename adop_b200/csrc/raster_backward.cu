@@ -16,6 +16,7 @@
 //  * the all-points kernels read the ghost stencil from one interleaved record per pixel [I_0..I_C-1, G_0..G_C-1] that a
 //    preparation pass builds (a neighbour then costs one or two 32-byte sectors instead of 2C).
 #include "common.cuh"
+#include "per_device.h"
 
 namespace adop {
 
@@ -1226,13 +1227,13 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
     const int want_geo = (bt.grad_points || bt.grad_pose || bt.grad_intrinsics) ? 1 : 0;
     const size_t smem = tile_smem_bytes(C, lt.L);
     const bool deep = lt.L > 4;
-    static size_t smem_set[2] = {0, 0};
-    if (smem > smem_set[deep])
-    {
-        if (deep) ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else ADOP_CUDA_TRY(cudaFuncSetAttribute(k_backward_tiles<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        smem_set[deep] = smem;
-    }
+    static OncePerDevice smem_set[2];  // (the kernel decides the size: one value for each)
+    int device = 0;
+    ADOP_CUDA_TRY(cudaGetDevice(&device));
+    ADOP_CUDA_TRY(smem_set[deep].run(device, [&] {
+        return deep ? cudaFuncSetAttribute(k_backward_tiles<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                    : cudaFuncSetAttribute(k_backward_tiles<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    }));
     int per_sm = 0;
     cudaError_t oe = deep ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, true>, kTileThreads, smem)
                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tiles<C, false>, kTileThreads, smem);

@@ -609,6 +609,32 @@ def test_struct_sizes_match_the_header():
     assert sizes == [ctypes.sizeof(m) for m in mirrors]
 
 
+def test_once_per_device_is_once_for_each_device():
+    """The helper behind attributes that belong to the current device (the tile kernel's shared memory): every device gets it, a
+    failure is tried again, and an unknown device number gets it on every call."""
+    import subprocess
+    import tempfile
+    src = r"""
+    #include <stdio.h>
+    #include "per_device.h"
+    int main()
+    {
+        static adop::OncePerDevice once;
+        int calls[3] = {0, 0, 0}, fail = 1;
+        for (int k = 0; k < 4; ++k)
+            for (int d = 0; d < 2; ++d) once.run(d, [&] { ++calls[d]; return 0; });
+        int first = once.run(2, [&] { return fail; }), second = once.run(2, [&] { return 0; }), third = once.run(2, [&] { return fail; });
+        for (int k = 0; k < 4; ++k) once.run(adop::OncePerDevice::kDevices + k % 2, [&] { ++calls[2]; return 0; });
+        printf("%d %d %d %d %d %d\n", calls[0], calls[1], first, second, third, calls[2]);
+        return 0;
+    }"""
+    with tempfile.TemporaryDirectory() as d:
+        open(os.path.join(d, "p.cpp"), "w").write(src)
+        subprocess.run(["/usr/bin/g++", "-std=c++17", "-I", os.path.join(ROOT, "adop_b200", "csrc"), os.path.join(d, "p.cpp"), "-o", os.path.join(d, "p")], check=True)
+        out = subprocess.run([os.path.join(d, "p")], capture_output=True, text=True).stdout
+    assert out.split() == ["1", "1", "1", "0", "0", "4"]
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(capi, "_lib", None)
     monkeypatch.setattr(capi, "LIB_PATH", "/nonexistent/libadop_raster.so")

@@ -404,6 +404,19 @@ def test_both_directions_run_on_a_part_of_the_gpu(cuda_lib, eight_sm_stream, cha
             close(b[k], whole[k].cpu().numpy(), name=f"eight SMs {name} {k}")
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_backward_on_a_second_device_of_the_process(cuda_lib):
+    """The tile kernel's shared-memory size is told to each device."""
+    cfg = synth.make_config("c2", n_points=20_000, n_views=2, size=(96, 64))
+    out = []
+    for dev in ("cuda:0", "cuda:1"):
+        scene, r = to_scene(cfg["arrays"], dev), PointRasterizer(dev)
+        grads = [torch.from_numpy(g).to(dev) for g in synth.upstream_gradients(cfg["meta"], batch=2)]
+        out.append(r.backward(scene, cfg["params"], r.forward(scene, cfg["views"], cfg["params"], 4), grads))
+    for k in ("texture", "points", "pose", "intrinsics"):
+        close(out[1][k], out[0][k].cpu().numpy(), name=f"second device {k}")
+
+
 def test_small_workspace_matches_full_workspace(cuda_lib):
     """With the full workspace the depth prepass hands projected points to the blend kernel; with the small one the blend
     kernel projects again. Same depth and weight bits, colours and gradients within the atomic-order tolerance."""
