@@ -230,7 +230,7 @@ __device__ __forceinline__ unsigned lanes_with_digit(unsigned digit)
 
 // Stable scatter of one tile (2048 keys) per block. Warp w owns keys [256 w, 256 w + 256) of the tile and keeps them in
 // registers (8 rounds of 32 consecutive keys). Three block-wide barriers per tile:
-//   1. every warp counts its digits (match.any per round, the lowest lane of each group adds the group size);
+//   1. every warp counts its digits (groups by votes, the lowest lane of each group adds the group size);
 //   2. thread d turns the per-warp counts of digit d into places inside the tile sorted by digit (tile prefix of the
 //      digit + warps before), and remembers where the tile's run of digit d starts in the output;
 //   3. every warp walks its rounds again (with the groups it found in step 1): place = its digit's place + keys of that

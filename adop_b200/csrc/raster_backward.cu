@@ -202,10 +202,11 @@ struct BackwardTargets
     float* grad_texture;
     float* grad_texture_interleaved;   // optional [T,C]; when set the descriptor gradient goes there
     float4* grad_points;
-    double* grad_pose;        // row of this view's image, 6 doubles
-    float* count_pose;        // element of this view's image
-    float* grad_intrinsics;   // row of this view's camera
-    float* count_intrinsics;  // element of this view's camera
+    // the tensors' first rows; a view's rows come from the table behind the camera records (ViewRows)
+    double* grad_pose;        // 6 doubles per image
+    float* count_pose;
+    float* grad_intrinsics;   // one row per camera
+    float* count_intrinsics;
 };
 
 // interleaved [I | G] of a pyramid pixel, written by the preparation pass
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(kBlock) k_splat_backward_all(PointStreams pts,
 //                   ONE work item for the chain kernel: the point's image-space ghost gradient summed over its layers,
 //                   each scaled by 0.5^layer (the projection chain is linear in that gradient, and a layer's crop
 //                   transform is the full-resolution one times 0.5^layer, PointRenderer.cu:616).
-//   k_chain_and_holes  one launch whose blocks split 3 : 1 between two independent parts: per work item, the summed
+//   k_chain_and_holes  one launch whose blocks split 5 : 3 between two independent parts: per work item, the summed
 //                   image-space gradient chained through the projection to the point, pose and intrinsics gradients
 //                   (block-reduced); and the background-colour and environment-map gradient of the uncovered pixels.
 // Nothing here waits on another block. These kernels are bound by memory latency, not by bandwidth or arithmetic: each
@@ -888,7 +889,7 @@ __device__ __forceinline__ void hole_gradients_part(const LayerTable& lt, int vi
 }
 
 // ---- per-point chain ---------------------------------------------------------------------------------------------------
-// A visible point with its summed image-space gradient, as parked in shared memory by k_point_chain.
+// A visible point with its summed image-space gradient, as parked in shared memory by point_chain_part.
 struct ChainItem
 {
     int id;

@@ -13,7 +13,8 @@
 //    (44 MB at 1080p with four channels) is reused by every view of the batch. It does not stay in L2 while a 10 M point
 //    cloud streams through: the blend kernel's L2 hit rate is about 40 %;
 //  * the blend kernel also lists, per 32 x 16 screen tile, the points the backward pass will visit, and the depth prepass can
-//    hand the blend kernel the projected in-image points (candidate streams) when the workspace has room for them.
+//    hand the blend kernel the projected points that can still be accepted (candidate streams) where that pays and the
+//    workspace has room for them.
 #include <cstring>
 
 #include "common.cuh"

@@ -48,9 +48,9 @@ def parse_args():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-c4", action="store_true", help="N > 1: skip the 30 M point record")
     ap.add_argument("--no-extras", action="store_true", help="N = 1: skip the tonemapper / Morton reorder record")
-    ap.add_argument("--candidates", action="store_true",
-                    help="size the scratch with room for candidate streams (the depth prepass then hands projected points to "
-                         "the blend kernel; measured slightly slower overall than projecting twice)")
+    ap.add_argument("--small-workspace", action="store_true",
+                    help="the small forward scratch: no candidate streams, no grouped accumulators (the default is what the call "
+                         "makes use of)")
     ap.add_argument("--no-touched", action="store_true",
                     help="N > 1: the exchange kernel reads every rank's whole gradient block instead of only the chunks a rank flagged")
     ap.add_argument("--exchange", default="peer", choices=["peer", "nccl"],
@@ -437,7 +437,7 @@ def main():
     w, h = cfg["meta"]["w"], cfg["meta"]["h"]
     P = sum(a * b for a, b in capi.layer_sizes(w, h, L))
     scene = Scene(**{k: (torch.from_numpy(v).to(dev) if v is not None else None) for k, v in arrays.items()})
-    ras = PointRasterizer(dev, full_workspace=True if args.candidates else None)
+    ras = PointRasterizer(dev, full_workspace=False if args.small_workspace else None)
     gen = torch.Generator(device=dev)
     gen.manual_seed(1234 + rank)
     grads_dev = [torch.randn((V, C, hh, ww), device=dev, generator=gen) for ww, hh in capi.layer_sizes(w, h, L)]

@@ -170,6 +170,21 @@ def test_knn_distance_in_uneven_surroundings(cuda_lib, n, shape):
     assert np.array_equal(got, _knn_brute_force(xyz, 4))
 
 
+@pytest.mark.parametrize("k", [4, 7])
+def test_knn_distance_with_a_crowded_cell(cuda_lib, k):
+    """5000 distinct points in the corner cell of a sparse cloud: more than the search's first way takes in one cell (2427), fewer
+    than a query may visit, so that every query of the cloud grows its cube. Exact values."""
+    rng = np.random.default_rng(k)
+    xyz = rng.uniform(0, 1, (6500, 3))
+    xyz[:5000] = rng.uniform(0, 1e-3, (5000, 3))
+    xyz = rng.permutation(xyz.astype(np.float32))
+    assert len(np.unique(xyz, axis=0)) == 6500
+    pos = np.zeros((6500, 4), np.float32)
+    pos[:, :3] = xyz
+    got = preprocess.knn_distance(torch.from_numpy(pos).cuda(), k=k).cpu().numpy()
+    assert np.array_equal(got, _knn_brute_force(xyz, k))
+
+
 def test_knn_distance_against_a_kd_tree(cuda_lib):
     """300 k points on surfaces (the benchmark's scene generator): scipy's KD-tree in float64 as the second opinion."""
     from scipy.spatial import cKDTree
