@@ -15,6 +15,8 @@
 //    are reduced warp -> block in shared memory and leave as one atomic per component and block;
 //  * the all-points kernels read the ghost stencil from one interleaved record per pixel [I_0..I_C-1, G_0..G_C-1] that a
 //    preparation pass builds (a neighbour then costs one or two 32-byte sectors instead of 2C).
+#include <algorithm>
+
 #include "common.cuh"
 #include "per_device.h"
 
@@ -1249,13 +1251,18 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
     const int hole_need = (ha.grad_env || ha.grad_background) ? (int)((groups + kBlock - 1) / kBlock) : 0;
     if (hole_need || want_geo)
     {
-        // the chain blocks get five eighths of the blocks when both parts have work (measured: between a half and three quarters
-        // the kernel's time is flat, beyond it rises quickly)
-        // A batch of two to four views gets twice the resident blocks: its views differ in work, and a block row that is done early
-    // leaves room for the next (chain and holes, one wave and two: four 4K views 1655 and 1495 us, sixteen 1080p views 856 and
-    // 869, eight 568 and 646, one 512 x 512 view 16.9 and 18.9).
-    const int per_view = blocks_per_view(g, views >= 2 && views <= 4 ? 2 : 1, views, 1 << 30);
-        int chain_blocks = want_geo ? (hole_need ? per_view * 5 / 8 : per_view) : 0;
+        // The resident blocks are shared out over the views, rounded down: a handful of blocks over that (three views, 198 x 3
+        // blocks in 592 places) run alone at the end, at twice the time (1080p, six million points: 336 us, rounded down 185). The chain
+        // blocks get five eighths of a view's blocks when both parts have work (between a half and three quarters the kernel's
+        // time is flat, beyond it rises quickly). Where a chain block would walk many tiles, which differ in their points, four times
+        // as many blocks even that out. One row of blocks : four, by tiles per chain block: 44 (1080p, four views) 254 : 277 us, 66 (six) 339 : 371,
+        // 78 (1280 x 720, sixteen) 372 : 371, 88 (1080p, eight; eight channels) 665 : 599, 177 (sixteen, four channels) 936 : 850, 176 (four at
+        // 4K, eight channels) 2134 : 1466.
+        const auto chain_share = [&](int blocks) { return want_geo ? (hole_need ? blocks * 5 / 8 : blocks) : 0; };
+        const int one_row = std::max(1, g / views);
+        const int rows_of_blocks = tt.n_tiles > 80 * std::max(1, chain_share(one_row)) ? 4 : 1;
+        const int per_view = std::max(1, g * rows_of_blocks / views);
+        int chain_blocks = chain_share(per_view);
         if (want_geo && chain_blocks < 1) chain_blocks = 1;
         if (chain_blocks > tt.n_tiles) chain_blocks = tt.n_tiles;
         int hole_blocks = per_view - chain_blocks < hole_need ? per_view - chain_blocks : hole_need;

@@ -568,6 +568,27 @@ def test_pose_gradient_of_a_batch_is_summed_in_double(cuda_lib):
     assert np.abs(off).max() <= 21 * 2.0 ** -24, off
 
 
+@pytest.mark.parametrize("views,size", [(3, (121, 83)), (64, (704, 320)), (70, (33, 17))])
+def test_chain_blocks_of_any_batch_cover_every_tile_and_hole(cuda_lib, views, size):
+    """Rows of chain and hole blocks: three views share the blocks unevenly; 64 views of 440 tiles have five chain blocks each in one row
+    and get four; 70 views (two chunks) of six tiles have fewer tiles than blocks. Against the views one by one."""
+    cfg = synth.make_config("c2", n_points=30_000, n_views=views, size=size, layers=3)
+    a, params, L = cfg["arrays"], cfg["params"], 3
+    scene = to_scene(a)
+    gen = torch.Generator(device="cuda:0").manual_seed(views)
+    grads = [torch.randn((views, 4, h, w), device="cuda:0", generator=gen) for w, h in capi.layer_sizes(*size, L)]
+    keys = ("texture", "background", "points", "pose", "intrinsics", "env_map", "count_pose", "count_intrinsics")
+    r, one = PointRasterizer("cuda:0"), PointRasterizer("cuda:0")
+    batch = r.backward(scene, params, r.forward(scene, cfg["views"], params, L), grads, want_env=True, normalize=False)
+    total = None
+    for b in range(views):
+        g = one.backward(scene, params, one.forward(scene, cfg["views"][b:b + 1], params, L), [x[b:b + 1].contiguous() for x in grads],
+                         want_env=True, normalize=False)
+        total = {k: g[k].double() + (total[k] if total else 0.0) for k in keys}
+    for k in keys:
+        close(batch[k], total[k].cpu().numpy(), name=f"chain rows {k}")
+
+
 def test_backward_mode_4(oracle, cuda_lib):
     cfg = synth.make_config("c1", n_points=40_000, size=(96, 96))
     cfg["params"].test_backward_mode = 4
