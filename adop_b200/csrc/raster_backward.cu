@@ -1260,7 +1260,7 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
         // 4K, eight channels) 2134 : 1466.
         const auto chain_share = [&](int blocks) { return want_geo ? (hole_need ? blocks * 5 / 8 : blocks) : 0; };
         const int one_row = std::max(1, g / views);
-        const int rows_of_blocks = tt.n_tiles > 80 * std::max(1, chain_share(one_row)) ? 4 : 1;
+        const int rows_of_blocks = tt.n_tiles > 80 * std::max(1, chain_share(one_row)) ? 4 : (views >= 2 && views <= 4 ? 2 : 1);
         const int per_view = std::max(1, g * rows_of_blocks / views);
         int chain_blocks = chain_share(per_view);
         if (want_geo && chain_blocks < 1) chain_blocks = 1;
