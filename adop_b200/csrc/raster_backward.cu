@@ -1258,6 +1258,9 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
         // as many blocks even that out. One row of blocks : four, by tiles per chain block: 44 (1080p, four views) 254 : 277 us, 66 (six) 339 : 371,
         // 78 (1280 x 720, sixteen) 372 : 371, 88 (1080p, eight; eight channels) 665 : 599, 177 (sixteen, four channels) 936 : 850, 176 (four at
         // 4K, eight channels) 2134 : 1466.
+        // Below that, two to four views keep two rows: crops of a training batch differ in their points, and blocks that are done early leave
+        // room for the next view's (four 512 x 512 crops, one row : two, whole step 428 : 409 us), though views that are alike lose by it
+        // (1080p, two views 136 : 160 us, four 254 : 268).
         const auto chain_share = [&](int blocks) { return want_geo ? (hole_need ? blocks * 5 / 8 : blocks) : 0; };
         const int one_row = std::max(1, g / views);
         const int rows_of_blocks = tt.n_tiles > 80 * std::max(1, chain_share(one_row)) ? 4 : (views >= 2 && views <= 4 ? 2 : 1);
