@@ -1259,7 +1259,7 @@ static adop_status launch_list_backward(const PointStreams& pts, const ViewCam* 
         // 78 (1280 x 720, sixteen) 372 : 371, 88 (1080p, eight; eight channels) 665 : 599, 177 (sixteen, four channels) 936 : 850, 176 (four at
         // 4K, eight channels) 2134 : 1466.
         // Below that, two to four views keep two rows: crops of a training batch differ in their points, and blocks that are done early leave
-        // room for the next view's (four 512 x 512 crops, whole step with one row 428 us, with two 409 - 417 us on different boxes), though views that are alike lose by it
+        // room for the next view's (four 512 x 512 crops, whole step with one row 428 us, with two 409 us), though views that are alike lose by it
         // (1080p, two views 136 : 160 us, four 254 : 268).
         const auto chain_share = [&](int blocks) { return want_geo ? (hole_need ? blocks * 5 / 8 : blocks) : 0; };
         const int one_row = std::max(1, g / views);
